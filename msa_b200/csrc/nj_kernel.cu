@@ -3,6 +3,10 @@
 // njoining::sequential<transform::linear<2>>
 // (src/phylogeny/njoining/impl/sequential.cpp:80-358).
 //
+// nj_join.cuh holds the kernels that a run uses; nj_cluster_kernel below is the
+// one that can spread a join's search over more clusters (msa_nj_set_clusters),
+// and runs only when the context asks for that.
+//
 // Layout. The reference keeps a packed symmetric matrix and, after every join,
 // swaps the removed OTU y with logical 0 and deletes logical 0
 // (src/phylogeny/matrix.cu:359-384, sequential.cpp:210-224); every index then
@@ -46,37 +50,16 @@
 #include <cstring>
 #include <vector>
 
-#include <cooperative_groups.h>
-
 #include "msa_internal.hpp"
+#include "nj_join.cuh"
 
 namespace msa {
 namespace njdev {
 
-namespace cg = cooperative_groups;
-
-constexpr unsigned kFull = 0xffffffffu;
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
-constexpr unsigned kMaxCluster = 16;
-constexpr uint32_t kNone = 0xffffffffu;
 // Row chunks (4 floats) each lane has in flight while scanning.
 constexpr int kBatch = 4;
-// Phase counters: CTA 0 (scan, wait at A, join, wait at B, writes) and the
-// folding CTA (fold, scan of the new node's row, wait at A).
-constexpr int kCycleSlots = 8;
-
-// Orderable key of a finite or +inf Q value; 0 for NaN and -inf, which the
-// reference's strict `q > best` (best starting at -inf) never selects.
-// -0 and +0 compare equal there, so both map to the +0 key.
-__device__ __forceinline__ uint32_t order_key(float q)
-{
-    if(q != q || q == -INFINITY) return 0u;
-    uint32_t b = __float_as_uint(q);
-    if(b == 0x80000000u) b = 0u;
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
 // Two float lanes in one 64-bit register and the packed float operations of
 // sm_100 on them: each lane is rounded to nearest as the scalar operation
 // (no flush to zero), so `sub2(sub2(mul2(a, b), c), d)` gives per lane the
@@ -104,31 +87,6 @@ __device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigne
     return r;
 }
 
-// A candidate pair (i, j), j < i, as one 64-bit key: larger Q wins; on equal
-// Q the pair earlier in the reference's row-major scan of the lower triangle
-// (smaller i, then smaller j) wins, which is the order of i << 16 | j (i, j <
-// 2^16). 0 means "no candidate"; the low word names the pair.
-__device__ __forceinline__ unsigned long long pack(uint32_t key, uint32_t i, uint32_t j)
-{
-    return key ? (((unsigned long long) key << 32) | (0xffffffffu - ((i << 16) | j))) : 0ull;
-}
-__device__ __forceinline__ uint32_t pair_of(unsigned long long v) { return 0xffffffffu - (uint32_t) v; }
-
-__device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
-
-// The warp's maximum of a 64-bit key in two 32-bit warp reductions: the
-// largest high word, then the largest low word among the lanes holding it.
-__device__ __forceinline__ unsigned long long warp_max(unsigned long long v)
-{
-    const uint32_t hi = (uint32_t) (v >> 32), lo = (uint32_t) v;
-    const uint32_t mhi = __reduce_max_sync(kFull, hi);
-    const uint32_t mlo = __reduce_max_sync(kFull, hi == mhi ? lo : 0u);
-    return ((unsigned long long) mhi << 32) | mlo;
-}
-
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
 struct State {
     float *D;                  // n rows of P floats; slot t + k holds logical k
     const float *S0;           // initial row sums by slot
@@ -152,14 +110,10 @@ struct State {
 };
 
 constexpr uint32_t kStop = 0xffffffffu;
-// Helper clusters: at most this many CTAs in all; kDefaultClusters - 1 of
-// them by default (none: on 2,000 OTUs, 3 helper clusters above 1,400 OTUs
-// measured 21.65 ms against 21.64 ms for one cluster, because the two
-// handoffs through global memory per join cost what the wider scan saves),
-// scanning while more than kHelperMinCount OTUs remain; every wait between
-// clusters ends after kWaitUs.
+// Helper clusters: at most this many CTAs in all, by default scanning while
+// more than kHelperMinCount OTUs remain; every wait between clusters ends
+// after kWaitUs. None run unless the context asks for them.
 constexpr uint32_t kMaxHelperCtas = 128;
-constexpr uint32_t kDefaultClusters = 1;
 constexpr uint32_t kHelperMinCount = 1400;
 constexpr uint32_t kWaitUs = 1000000;
 
@@ -444,9 +398,7 @@ __device__ void nj_helper(const State &st, float *S, uint32_t hidx, uint32_t sid
     }
 }
 
-// kHelp: the launch has helper clusters (compiled separately, so that the
-// one-cluster kernel carries none of their code).
-template <bool Linear, bool kHelp>
+template <bool Linear>
 __global__ void __launch_bounds__(kThreads, 1) nj_cluster_kernel(State st)
 {
     cg::cluster_group cluster = cg::this_cluster();
@@ -476,12 +428,10 @@ __global__ void __launch_bounds__(kThreads, 1) nj_cluster_kernel(State st)
     const unsigned K = cluster.num_blocks();
     const unsigned rank = cluster.block_rank();
     const unsigned F = K - 1;   // the CTA that folds new row sums
-    if constexpr(kHelp) {
-        if(blockIdx.x >= K) {       // a helper cluster
-            nj_helper<Linear>(st, reinterpret_cast<float *>(smem_raw), blockIdx.x - K, F + blockIdx.x - K,
-                              F + st.helper_ctas);
-            return;
-        }
+    if(blockIdx.x >= K) {       // a helper cluster
+        nj_helper<Linear>(st, reinterpret_cast<float *>(smem_raw), blockIdx.x - K, F + blockIdx.x - K,
+                          F + st.helper_ctas);
+        return;
     }
     const bool folder = rank == F;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -527,7 +477,7 @@ __global__ void __launch_bounds__(kThreads, 1) nj_cluster_kernel(State st)
     while(c > 1) {
         const float cm2 = (float) (c - 2);
         // The helper clusters scan with cluster 0 for this join.
-        const bool helped = kHelp && st.helper_ctas != 0u && !hoff && c > st.helper_c;
+        const bool helped = st.helper_ctas != 0u && !hoff && c > st.helper_c;
         unsigned long long best = 0;
 
         // ---- scan
@@ -569,7 +519,7 @@ __global__ void __launch_bounds__(kThreads, 1) nj_cluster_kernel(State st)
             const unsigned long long v = lane < kWarps ? wbest[lane] : 0ull;
             unsigned long long m = warp_max(v);
             int off = 0;
-            if(kHelp && rank == 0 && helped) {
+            if(rank == 0 && helped) {
                 // The helper CTAs' candidates for this join, each lane waiting
                 // for its share of them; merged into this CTA's part.
                 const uint32_t buf = step & 1u;
@@ -670,7 +620,7 @@ __global__ void __launch_bounds__(kThreads, 1) nj_cluster_kernel(State st)
             if(tid == 0 && mv) S[t + y] = S[t + src];
             // The row sums after this join and the joined pair, for the helper
             // clusters' next scan (this CTA's copy has no +inf masks).
-            if(kHelp && st.helper_ctas != 0u && !hoff && c - 1 > st.helper_c) {
+            if(st.helper_ctas != 0u && !hoff && c - 1 > st.helper_c) {
                 __syncthreads();   // update_cache above
                 const uint32_t buf = step & 1u;
                 float *pub = st.s_pub + (size_t) buf * P;
@@ -859,7 +809,7 @@ __global__ void __launch_bounds__(kThreads, 1) nj_cluster_kernel(State st)
     if(failed && rank == 0 && tid == 0) atomicExch(st.err, 2);
     if(bad && rank == 0 && tid == 0) atomicExch(st.err, 4);
     // Helpers still waiting for a publication stop.
-    if(kHelp && folder && tid == 0 && st.helper_ctas != 0u && !st.stall_publication) st_release(st.pub_seq, kStop);
+    if(folder && tid == 0 && st.helper_ctas != 0u && !st.stall_publication) st_release(st.pub_seq, kStop);
     if(tid == 0 && rank == 0)
         for(int k = 0; k < 5; ++k) st.cycles[k] = cyc[k];
     if(tid == 0 && folder)
@@ -867,41 +817,19 @@ __global__ void __launch_bounds__(kThreads, 1) nj_cluster_kernel(State st)
     cluster.sync();   // no CTA leaves while another may still write its shared memory
 }
 
-// Packed triangle (float or int32) -> full symmetric matrix of pitch P,
-// diagonal and padding 0.
-template <class T>
-__global__ void inflate_kernel(const T *__restrict__ tri, float *__restrict__ D, uint32_t n, uint32_t P)
-{
-    const uint64_t total = (uint64_t) n * P;
-    for(uint64_t e = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t) gridDim.x * blockDim.x) {
-        const uint64_t i = e / P, j = e - i * P;
-        float v = 0.0f;
-        if(j < n) {
-            if(i > j) v = (float) tri[i * (i - 1) / 2 + j];
-            else if(j > i) v = (float) tri[j * (j - 1) / 2 + i];
-        }
-        D[e] = v;
-    }
-}
-
-// cache_init (sequential.cpp:80-94): S[k] folds D[k][j] over j != k ascending,
-// from 0. Thread k reads column k (= row k by symmetry) so a warp's reads coalesce.
-__global__ void row_sums_kernel(const float *__restrict__ D, float *__restrict__ S, uint32_t n, uint32_t P)
-{
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if(k >= n) return;
-    float s = 0.0f;
-    for(uint32_t j = 0; j < n; ++j)
-        if(j != k) s = __fadd_rn(s, D[(size_t) j * P + k]);
-    S[k] = s;
-}
-
-// Largest cluster (16, 8, 4 or 2 CTAs) that can be resident with `smem` bytes
-// of dynamic shared memory per CTA; 0 if none.
-template <bool Linear, bool kHelp>
-unsigned pick_cluster(size_t smem)
+// Largest cluster (16, 8, 4 or 2 CTAs) of `kern` that can be resident with
+// smem(k) bytes of dynamic shared memory per CTA, and how many of them; 0 if none.
+template <class Kern, class Smem>
+unsigned pick_cluster(Kern kern, unsigned threads, Smem smem, int *clusters)
 {
     for(unsigned k : {16u, 8u, 4u, 2u}) {
+        const size_t bytes = smem(k);
+        if(bytes > kMaxSmem) continue;
+        if(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes) != cudaSuccess ||
+           cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -909,151 +837,218 @@ unsigned pick_cluster(size_t smem)
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         cfg.gridDim = dim3(k);
-        cfg.blockDim = dim3(kThreads);
-        cfg.dynamicSmemBytes = smem;
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = bytes;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        int clusters = 0;
-        if(cudaOccupancyMaxActiveClusters(&clusters, nj_cluster_kernel<Linear, kHelp>, &cfg) == cudaSuccess &&
-           clusters >= 1)
-            return k;
+        *clusters = 0;
+        if(cudaOccupancyMaxActiveClusters(clusters, kern, &cfg) == cudaSuccess && *clusters >= 1) return k;
         cudaGetLastError();
     }
     return 0;
 }
 
-}  // namespace njdev
-
-int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, msa_otu *out)
+template <class Kern, class Arg>
+cudaError_t launch_clusters(Kern kern, unsigned k, unsigned ctas, unsigned threads, size_t smem, cudaStream_t s,
+                            const Arg &arg)
 {
-    const bool linear = order == MSA_NJ_LINEAR;
-    auto kern_one = linear ? njdev::nj_cluster_kernel<true, false> : njdev::nj_cluster_kernel<false, false>;
-    auto kern_help = linear ? njdev::nj_cluster_kernel<true, true> : njdev::nj_cluster_kernel<false, true>;
-    cudaStream_t s = ctx->stream;
-    const uint32_t P = (n + 3) & ~3u;
-    const size_t smem = (size_t) P * 16;   // S, ND (4 B each), U (8 B)
-    if(n > 12800) return set_error(ctx, MSA_ERR_TOO_LARGE, "neighbor-joining supports at most 12800 OTUs");
-    const uint64_t ntri = (uint64_t) n * (n - 1) / 2;
-
-    // Device layout.
-    size_t off = 0;
-    auto take = [&off](size_t b) { size_t o = off; off = round_up(off + b, 256); return o; };
-    const size_t oD = take((size_t) n * P * 4), oS = take(n * 4), oRx = take(n * 4), oRy = take(n * 4),
-                 oRdx = take(n * 4), oRdy = take(n * 4), oErr = take(64), oCyc = take(64),
-                 oTri = take((kind == MSA_TRI_F32_HOST || kind == MSA_TRI_I32_HOST) ? ntri * 4 : 0),
-                 oPub = take((size_t) 2 * P * 4),
-                 // flags between clusters: pub_seq, pub_xy[2], cand_seq[], cand[][][2]
-                 oSync = take(64 + (size_t) njdev::kMaxHelperCtas * 4),
-                 oCand = take((size_t) 2 * njdev::kMaxHelperCtas * 16);
-    MSA_CUDA_TRY(ctx, ctx->nj_buf.ensure(off));
-    char *base = (char *) ctx->nj_buf.ptr;
-    njdev::State st{};
-    st.D = (float *) (base + oD);
-    st.S0 = (const float *) (base + oS);
-    st.rec_x = (uint32_t *) (base + oRx);
-    st.rec_y = (uint32_t *) (base + oRy);
-    st.rec_dx = (float *) (base + oRdx);
-    st.rec_dy = (float *) (base + oRdy);
-    st.err = (int *) (base + oErr);
-    st.cycles = (unsigned long long *) (base + oCyc);
-    st.n = n;
-    st.P = P;
-
-    for(auto kf : {kern_one, kern_help}) {
-        MSA_CUDA_TRY(ctx, cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-        MSA_CUDA_TRY(ctx, cudaFuncSetAttribute(kf, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    }
-    const unsigned K = linear ? njdev::pick_cluster<true, false>(smem) : njdev::pick_cluster<false, false>(smem);
-    if(K < 2) return set_error(ctx, MSA_ERR_CUDA, "neighbor-joining cluster cannot be resident");
-    // Helper clusters: as many as can be resident beside cluster 0 (each on
-    // its own GPC), at most the context's setting, and only when some join
-    // has more OTUs than the helpers' threshold.
-    const uint32_t helper_c = std::max<uint32_t>(ctx->nj_helper_c ? ctx->nj_helper_c : njdev::kHelperMinCount, 2);
-    uint32_t clusters = 1;
-    if(ctx->nj_clusters != 1 && n > helper_c + 1) {
-        cudaLaunchConfig_t q = {};
-        cudaLaunchAttribute qa[1];
-        qa[0].id = cudaLaunchAttributeClusterDimension;
-        qa[0].val.clusterDim.x = K;
-        qa[0].val.clusterDim.y = 1;
-        qa[0].val.clusterDim.z = 1;
-        q.gridDim = dim3(K);
-        q.blockDim = dim3(njdev::kThreads);
-        q.dynamicSmemBytes = smem;
-        q.attrs = qa;
-        q.numAttrs = 1;
-        int resident = 0;
-        if(cudaOccupancyMaxActiveClusters(&resident, kern_help, &q) != cudaSuccess) {
-            cudaGetLastError();
-            resident = 1;
-        }
-        const uint32_t want = ctx->nj_clusters ? (uint32_t) ctx->nj_clusters : njdev::kDefaultClusters;
-        clusters = std::max<uint32_t>(1, std::min<uint32_t>({want, (uint32_t) resident,
-                                                              1 + njdev::kMaxHelperCtas / K}));
-    }
-    auto kern = clusters > 1 ? kern_help : kern_one;
-    char *sync = base + oSync;
-    st.helper_ctas = (clusters - 1) * K;
-    st.helper_c = helper_c;
-    st.s_pub = (float *) (base + oPub);
-    st.pub_seq = (uint32_t *) sync;
-    st.pub_xy = (uint32_t *) (sync + 16);
-    st.cand_seq = (uint32_t *) (sync + 64);
-    st.cand = (unsigned long long *) (base + oCand);
-    st.wait_ns = (unsigned long long) (ctx->nj_wait_us ? ctx->nj_wait_us : njdev::kWaitUs) * 1000ull;
-    st.stall_publication = ctx->nj_stall;
-
-    MSA_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[0], s));
-    const void *dtri = tri;
-    if(kind == MSA_TRI_F32_HOST || kind == MSA_TRI_I32_HOST) {
-        MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + oTri, tri, ntri * 4, cudaMemcpyHostToDevice, s));
-        dtri = base + oTri;
-    }
-    const unsigned ib = (unsigned) std::min<uint64_t>(((uint64_t) n * P + 255) / 256, 65535);
-    if(kind == MSA_TRI_F32_HOST || kind == MSA_TRI_F32_DEVICE)
-        njdev::inflate_kernel<float><<<ib, 256, 0, s>>>((const float *) dtri, st.D, n, P);
-    else
-        njdev::inflate_kernel<int32_t><<<ib, 256, 0, s>>>((const int32_t *) dtri, st.D, n, P);
-    MSA_CUDA_TRY(ctx, cudaGetLastError());
-    njdev::row_sums_kernel<<<(n + 255) / 256, 256, 0, s>>>(st.D, (float *) (base + oS), n, P);
-    MSA_CUDA_TRY(ctx, cudaGetLastError());
-    MSA_CUDA_TRY(ctx, cudaMemsetAsync(base + oErr, 0, 64, s));
-    // Joins the kernel never records stay invalid (0xffffffff) and are caught
-    // before the tree is built.
-    MSA_CUDA_TRY(ctx, cudaMemsetAsync(base + oRx, 0xff, (size_t) n * 4, s));
-    MSA_CUDA_TRY(ctx, cudaMemsetAsync(base + oRy, 0xff, (size_t) n * 4, s));
-    MSA_CUDA_TRY(ctx, cudaMemsetAsync(base + oCyc, 0, 64, s));
-    MSA_CUDA_TRY(ctx, cudaMemsetAsync(sync, 0, 64 + (size_t) njdev::kMaxHelperCtas * 4, s));
-    ctx->launches += 2;
-
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = K;
+    attr[0].val.clusterDim.x = k;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(K * clusters);
-    cfg.blockDim = dim3(njdev::kThreads);
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    MSA_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[1], s));
-    MSA_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kern, st));
-    MSA_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[2], s));
-    ctx->launches++;
-    unsigned long long cyc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    return cudaLaunchKernelEx(&cfg, kern, arg);
+}
 
-    std::vector<uint32_t> rx(n - 1), ry(n - 1);
-    std::vector<float> rdx(n - 1), rdy(n - 1);
-    int err = 0;
-    MSA_CUDA_TRY(ctx, cudaMemcpyAsync(rx.data(), st.rec_x, (n - 1) * 4, cudaMemcpyDeviceToHost, s));
-    MSA_CUDA_TRY(ctx, cudaMemcpyAsync(ry.data(), st.rec_y, (n - 1) * 4, cudaMemcpyDeviceToHost, s));
-    MSA_CUDA_TRY(ctx, cudaMemcpyAsync(rdx.data(), st.rec_dx, (n - 1) * 4, cudaMemcpyDeviceToHost, s));
-    MSA_CUDA_TRY(ctx, cudaMemcpyAsync(rdy.data(), st.rec_dy, (n - 1) * 4, cudaMemcpyDeviceToHost, s));
-    MSA_CUDA_TRY(ctx, cudaMemcpyAsync(&err, st.err, 4, cudaMemcpyDeviceToHost, s));
-    MSA_CUDA_TRY(ctx, cudaMemcpyAsync(cyc, st.cycles, sizeof(cyc), cudaMemcpyDeviceToHost, s));
+// ... and up to this many run on four warps, whose steps per join cost less
+// than a wider search saves.
+constexpr uint32_t kTinyNodes = 64;
+// A launch joins until this share of its nodes is left, then the live ones
+// are packed into a smaller matrix: a search reads the slots of joined nodes
+// too, and each packing costs one search of the whole smaller matrix.
+constexpr double kStageShare = 0.6;
+
+}  // namespace njdev
+
+int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, msa_otu *out)
+{
+    using namespace njdev;
+    const bool linear = order == MSA_NJ_LINEAR;
+    cudaStream_t s = ctx->stream;
+    const bool on_host = kind == MSA_TRI_F32_HOST || kind == MSA_TRI_I32_HOST;
+    const bool is_int = kind == MSA_TRI_I32_HOST || kind == MSA_TRI_I32_DEVICE;
+    auto pitch = [](uint32_t m) { return (m + 4) & ~3u; };   // m + 1 slots
+    const uint32_t P = pitch(n);
+    if(n > 12800) return set_error(ctx, MSA_ERR_TOO_LARGE, "neighbor-joining supports at most 12800 OTUs");
+    const uint64_t ntri = (uint64_t) n * (n - 1) / 2;
+
+    // Clusters that scan beside the joining one, when the context asks for
+    // them (msa_nj_set_clusters) and some join has more OTUs than the
+    // helpers' threshold: the kernel with helpers runs the whole call.
+    const uint32_t helper_c = std::max<uint32_t>(ctx->nj_helper_c ? ctx->nj_helper_c : kHelperMinCount, 2);
+    auto kern_help = linear ? nj_cluster_kernel<true> : nj_cluster_kernel<false>;
+    auto kern_join = linear ? nj_join_kernel<true> : nj_join_kernel<false>;
+    const size_t help_smem = (size_t) P * 16;   // S, ND (4 B each), U (8 B)
+    unsigned K = 1;
+    uint32_t clusters = 1;
+    bool helped = false;
+    if(ctx->nj_clusters > 1 && n > helper_c + 1) {
+        int resident = 0;
+        K = pick_cluster(kern_help, kThreads, [&](unsigned) { return help_smem; }, &resident);
+        if(K < 2) return set_error(ctx, MSA_ERR_CUDA, "neighbor-joining cluster cannot be resident");
+        clusters = std::max<uint32_t>(1, std::min<uint32_t>({(uint32_t) ctx->nj_clusters, (uint32_t) resident,
+                                                              1 + kMaxHelperCtas / K}));
+        helped = clusters > 1;
+    }
+    if(!helped && n > kSmallNodes) {
+        int resident = 0;
+        K = pick_cluster(kern_join, kJoinThreads, [&](unsigned k) { return join_smem(P, (n + k) / k); },
+                         &resident);
+        if(K < 2) {
+            // Too many rows per CTA for the row states of a small cluster: the
+            // kernel with (here no) helpers needs no state per row.
+            K = pick_cluster(kern_help, kThreads, [&](unsigned) { return help_smem; }, &resident);
+            if(K < 2) return set_error(ctx, MSA_ERR_CUDA, "neighbor-joining cluster cannot be resident");
+            helped = true;
+        }
+    }
+
+    // The launches' node counts.
+    std::vector<uint32_t> stages{n};
+    while(!helped && stages.back() > kSmallNodes)
+        stages.push_back(std::max<uint32_t>(kSmallNodes, (uint32_t) (stages.back() * kStageShare)));
+    const bool direct = !helped && n <= kSmallNodes;   // the launch reads the triangle itself
+    const uint32_t n2 = stages.size() > 1 ? stages[1] : 0;
+
+    // Device layout. Everything the host reads back is one run of words from oHead.
+    size_t off = 0;
+    auto take = [&off](size_t b) { size_t o = off; off = round_up(off + b, 256); return o; };
+    const size_t oHead = take(256), oRec = take((size_t) n * 16), oS = take((size_t) P * 4), oS2 = take((size_t) P * 4),
+                 oOrd = take((size_t) n * 4), oD = take(direct ? 0 : (size_t) (n + 1) * P * 4),
+                 oD2 = take(n2 ? (size_t) (n2 + 1) * pitch(n2) * 4 : 0), oTri = take(on_host ? ntri * 4 : 0),
+                 oPub = take(helped ? (size_t) 2 * P * 4 : 0),
+                 // flags between clusters: pub_seq, pub_xy[2], cand_seq[], cand[][][2]
+                 oSync = take(helped ? 64 + (size_t) kMaxHelperCtas * 4 : 0),
+                 oCand = take(helped ? (size_t) 2 * kMaxHelperCtas * 16 : 0);
+    MSA_CUDA_TRY(ctx, ctx->nj_buf.ensure(off));
+    char *base = (char *) ctx->nj_buf.ptr;
+    // Head: phase counters, the error word, the largest |D|.
+    unsigned long long *d_cycles = (unsigned long long *) (base + oHead);
+    int *d_err = (int *) (base + oHead + 64);
+    uint32_t *d_mabs = (uint32_t *) (base + oHead + 68);
+    uint32_t *rec = (uint32_t *) (base + oRec);
+    float *rec_f = (float *) (base + oRec);
+
+    MSA_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[0], s));
+    // Joins the kernels never record stay invalid (0xffffffff) and are caught
+    // before the tree is built.
+    MSA_CUDA_TRY(ctx, cudaMemsetAsync(base + oHead, 0, 128, s));
+    MSA_CUDA_TRY(ctx, cudaMemsetAsync(rec, 0xff, (size_t) n * 16, s));
+    const void *dtri = tri;
+    if(on_host) {
+        MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + oTri, tri, ntri * 4, cudaMemcpyHostToDevice, s));
+        dtri = base + oTri;
+    }
+    if(!direct) {
+        const dim3 tiles((P + 31) / 32, (P + 31) / 32);
+        float *D = (float *) (base + oD);
+        if(is_int) inflate_kernel<int32_t><<<tiles, 256, 0, s>>>((const int32_t *) dtri, D, n, P, d_mabs);
+        else inflate_kernel<float><<<tiles, 256, 0, s>>>((const float *) dtri, D, n, P, d_mabs);
+        MSA_CUDA_TRY(ctx, cudaGetLastError());
+        row_sums_kernel<<<(n + 31) / 32, 32, 0, s>>>(D, (float *) (base + oS), n, P);
+        MSA_CUDA_TRY(ctx, cudaGetLastError());
+        ctx->launches += 2;
+    }
+
+    if(helped) {
+        State st{};
+        st.D = (float *) (base + oD);
+        st.S0 = (const float *) (base + oS);
+        st.rec_x = rec;
+        st.rec_y = rec + n;
+        st.rec_dx = rec_f + 2 * (size_t) n;
+        st.rec_dy = rec_f + 3 * (size_t) n;
+        st.err = d_err;
+        st.cycles = d_cycles;
+        st.n = n;
+        st.P = P;
+        char *sync = base + oSync;
+        st.helper_ctas = (clusters - 1) * K;
+        st.helper_c = helper_c;
+        st.s_pub = (float *) (base + oPub);
+        st.pub_seq = (uint32_t *) sync;
+        st.pub_xy = (uint32_t *) (sync + 16);
+        st.cand_seq = (uint32_t *) (sync + 64);
+        st.cand = (unsigned long long *) (base + oCand);
+        st.wait_ns = (unsigned long long) (ctx->nj_wait_us ? ctx->nj_wait_us : kWaitUs) * 1000ull;
+        st.stall_publication = ctx->nj_stall;
+        MSA_CUDA_TRY(ctx, cudaMemsetAsync(sync, 0, 64 + (size_t) kMaxHelperCtas * 4, s));
+        MSA_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[1], s));
+        MSA_CUDA_TRY(ctx, launch_clusters(kern_help, K, K * clusters, kThreads, help_smem, s, st));
+        ctx->launches++;
+    } else {
+        MSA_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[1], s));
+        float *D = (float *) (base + oD), *D2 = (float *) (base + oD2);
+        float *S = (float *) (base + oS), *S2 = (float *) (base + oS2);
+        uint32_t *ord = (uint32_t *) (base + oOrd);
+        for(size_t k = 0; k < stages.size(); ++k) {
+            Stage st{};
+            st.N = stages[k];
+            st.P = pitch(st.N);
+            st.c_end = k + 1 < stages.size() ? stages[k + 1] : 1;
+            st.step0 = n - st.N;
+            st.D = D;
+            st.S0 = S;
+            st.S_out = S2;
+            st.order_out = ord;
+            st.mabs = d_mabs;
+            st.rec_x = rec;
+            st.rec_y = rec + n;
+            st.rec_dx = rec_f + 2 * (size_t) n;
+            st.rec_dy = rec_f + 3 * (size_t) n;
+            st.err = d_err;
+            st.cycles = d_cycles;
+            st.tri = direct ? dtri : nullptr;
+            st.tri_int = is_int;
+            if(st.N > kSmallNodes) {
+                MSA_CUDA_TRY(ctx, launch_clusters(kern_join, K, K, kJoinThreads,
+                                                  join_smem(st.P, (st.N + K) / K), s, st));
+                const uint32_t m = st.c_end;
+                compact_kernel<<<std::min<uint32_t>(m + 1, 4 * (uint32_t) ctx->num_sms), 256, 0, s>>>(
+                    D, st.P, ord, D2, m, pitch(m), d_err);
+                MSA_CUDA_TRY(ctx, cudaGetLastError());
+                std::swap(D, D2);
+                std::swap(S, S2);
+                ctx->launches += 2;
+            } else {
+                const size_t bytes = small_smem(st.N, st.P);
+                const int threads = st.N <= kTinyNodes ? 128 : 512;
+                auto kern_small = st.N <= kTinyNodes ? (linear ? nj_small_kernel<true, 128> : nj_small_kernel<false, 128>)
+                                                     : (linear ? nj_small_kernel<true, 512> : nj_small_kernel<false, 512>);
+                MSA_CUDA_TRY(ctx, cudaFuncSetAttribute(kern_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes));
+                kern_small<<<1, threads, bytes, s>>>(st);
+                MSA_CUDA_TRY(ctx, cudaGetLastError());
+                ctx->launches++;
+            }
+        }
+    }
+    MSA_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[2], s));
+    std::vector<uint32_t> back(64 + 4 * (size_t) n);   // head and records
+    MSA_CUDA_TRY(ctx, cudaMemcpyAsync(back.data(), base + oHead, back.size() * 4, cudaMemcpyDeviceToHost, s));
     MSA_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+    const uint32_t *rx = back.data() + 64, *ry = rx + n;
+    const float *rdx = (const float *) (ry + n), *rdy = rdx + n;
+    unsigned long long cyc[8];
+    int err = 0;
+    std::memcpy(cyc, back.data(), sizeof(cyc));
+    std::memcpy(&err, back.data() + 16, sizeof(err));
     {
         msa_nj_stats ns{};
         float ms = 0, ms_all = 0;

@@ -213,7 +213,8 @@ typedef struct msa_nw_stats {
     uint64_t cells;         /* sum over pairs of (effective rows x effective columns) */
     uint64_t pairs;
     uint32_t launches;      /* kernel launches issued by the call */
-    uint32_t narrow_tasks;  /* tasks run on 16-bit lanes */
+    uint32_t narrow_tasks;  /* tasks whose values fit 16-bit lanes as they are (longer ones run
+                               on 16-bit lanes relative to a moving base, or on 32-bit lanes) */
     uint32_t graph;         /* 1 if the call replayed a captured CUDA graph */
 } msa_nw_stats;
 int msa_nw_last_stats(const msa_ctx *ctx, msa_nw_stats *out);

@@ -355,7 +355,29 @@ struct JobView {
 
 // row_narrow flags: 16-bit lanes; rows pairs k and k + 1 stacked in one warp
 // (quad_task), their tasks all under k.
-constexpr uint8_t kRowNarrow = 1, kRowQuad = 2;
+// Rows pairs of several strips: kRowLong runs its 16-bit lanes on a moving base
+// (sweep_long), kRowChain makes every strip a task of its own, of 32 x 32, 16 or
+// 8 rows (chain_rows).
+constexpr uint8_t kRowNarrow = 1, kRowQuad = 2, kRowLong = 4, kRowChain = 8, kRowR16 = 16, kRowR8 = 32;
+
+// Steps between moves of a long strip's base; see sweep_long.
+constexpr int kRebase = 512;
+// Columns between two publications of a chained strip's progress.
+constexpr int kPublish = 64;
+// A chained strip waits at most this long for the one above it.
+constexpr unsigned long long kChainWaitNs = 5000000000ull;
+// Entries of a boundary row's base table for ncols columns, and the tables it
+// has: strip s writes table s mod 8 and reads the one before. A chained strip is
+// at least 128 steps behind the one it follows when it moves its base, so the
+// strip that writes a table again, 8 on, is 896 steps behind the last reader of
+// an entry that serves 512 columns.
+__host__ __device__ __forceinline__ uint32_t base_entries(uint32_t ncols) { return (ncols + 31) / kRebase + 2; }
+constexpr uint32_t kBaseTables = 8;
+// Words of a boundary row and its base tables.
+__host__ __device__ __forceinline__ uint64_t bound_words(uint32_t ncols)
+{
+    return ((uint64_t) ncols + 160 + 2 * kBaseTables * base_entries(ncols) + 31) / 32 * 32;
+}
 
 struct BatchParams {
     JobView job;
@@ -367,6 +389,14 @@ struct BatchParams {
     uint32_t *bound;
     uint64_t bound_stride;
     unsigned long long *counter;
+    // Chained rows pairs (the first ones of the launch): boundary rows of rows
+    // pair k, group g, warp w at chain_bound + chain_off[k] + (g W + w) words;
+    // progress of task q, warp w at chain_flag[(q - task_base) W + w].
+    uint32_t *chain_bound;
+    const uint64_t *chain_off;
+    uint32_t *chain_flag;
+    int *err;                   // set when a wait between strips ran out
+    uint32_t step;              // largest s + 2g, for the moving base
 };
 
 // Merged launches of the serving loop: explicit (job slot, rows pair, column
@@ -692,6 +722,186 @@ __device__ __forceinline__ typename K::W pick_row(const typename K::W (&H)[R], i
     return v;
 }
 
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p)
+{
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(uint32_t *p, uint32_t v)
+{
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// The strip above a chained one: its progress (columns of its last row that
+// may be read) and where this strip publishes its own; null where there is none.
+struct Chain {
+    const uint32_t *above;
+    uint32_t *mine;
+    int *err;
+};
+
+// Waits until *flag >= want and returns its value, or gives up: then, and in
+// every later wait of the launch, the strip runs on with what is there and the
+// call fails.
+__device__ __noinline__ uint32_t chain_wait(const uint32_t *flag, uint32_t want, int *err)
+{
+    unsigned long long t0, t1;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    for(;;) {
+        const uint32_t v = ld_acquire(flag);
+        if(v >= want) return v;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+        if(*(volatile int *) err != 0) return want;
+        if(t1 - t0 > kChainWaitNs) {
+            atomicExch(err, 1);
+            return want;
+        }
+        __nanosleep(100);
+    }
+}
+
+// sweep_strip for strips whose T outgrows 16 bits, and for chained strips: the
+// lanes hold T minus a base of the warp (one per 16-bit half), moved up every
+// kRebase steps by the smallest first-row value of the 32 lanes less one step.
+// T grows along rows and columns by at most `step` = smax + 2g per cell, so the
+// cells in flight (32R rows, 32 columns) and all that a lane can still read lie
+// within (32R + 33) step above that, and grow by kRebase step until the next
+// move: long_ok keeps the sum within 16 bits, whatever the sequences' lengths.
+// A boundary word is relative to its writer's base at the step that wrote it
+// (column j: step j + 31), which the writer leaves in tab_out and its reader
+// finds in tab_in.
+// 24 genomes of 30,000 bases: 334 ms in 32-bit lanes with all 30 strips of a
+// column in one warp (42 tasks on 296 resident CTAs), 27.9 ms with moving bases
+// and a task per strip; 50 genomes of 2,000 to 10,000 bases 15.8 -> 4.7 ms.
+template <int R, bool kPack>
+__device__ __forceinline__ void sweep_long(const uint32_t *__restrict__ sprof, const uint8_t *__restrict__ cols,
+                                           int ncols, uint32_t *bound, const int2 *tab_in, int2 *tab_out,
+                                           bool first, int tend,
+                                           bool store_bound, const Chain &chain, uint32_t step, int lane,
+                                           Narrow::W (&H)[R], int2 &base)
+{
+    using W = Narrow::W;
+    using L = Layout<R, true, kPack>;
+    constexpr int SH = L::SH;
+#pragma unroll
+    for(int r = 0; r < R; ++r) H[r] = 0u;   // column 0 of T
+    W diag = 0u, hlast = 0u;
+    base = make_int2(0, 0);
+    // Columns c0 + lane of the row above, relative to this warp's base. The
+    // progress above is read again only when the last value read falls short.
+    uint32_t known = 0;
+    auto load_above = [&](int c0) -> uint32_t {
+        if(first) return 0u;
+        if(chain.above) {
+            const uint32_t want = (uint32_t) min(c0 + 32, ncols);
+            if(known < want) known = chain_wait(chain.above, want, chain.err);
+        }
+        const int c = c0 + lane;
+        if(c >= ncols) return 0u;
+        const uint32_t w = __ldcg(bound + c);
+        const int2 b = __ldcg(tab_in + (c + 31) / kRebase);
+        return __vadd2(w, ((uint32_t) (b.x - base.x) & 0xffffu) | ((uint32_t) (b.y - base.y) << 16));
+    };
+    uint32_t bq_cur = load_above(0), bq_nxt = load_above(32);
+    const uint32_t *prow = sprof + lane * 4;
+    const int half_off = L::HALF - lane * 2, phalf_off = L::PHALF - lane * 2;
+    const bool st31 = store_bound && lane == 31;
+    __syncwarp();
+    if(st31) tab_out[0] = base;
+    int j = -lane;
+    uint32_t cur = cols[j], nxt = cols[j + 1];
+
+    auto group = [&](int t0, auto guard) {
+        constexpr bool kG = decltype(guard)::value;
+        if((t0 & 31) == 0 && t0 > 0) {
+            bq_cur = bq_nxt;
+            if(t0 % kRebase == 0) {
+                // Unsigned halves: the smallest H[0] of the lanes, less one step.
+                const uint32_t lo = __reduce_min_sync(kFull, H[0] & 0xffffu), hi = __reduce_min_sync(kFull, H[0] >> 16);
+                const uint32_t dlo = lo > step ? lo - step : 0u, dhi = hi > step ? hi - step : 0u;
+                const uint32_t d = dlo | dhi << 16;
+#pragma unroll
+                for(int r = 0; r < R; ++r) H[r] = __vsub2(H[r], d);
+                diag = __vsub2(diag, d);
+                hlast = __vsub2(hlast, d);
+                bq_cur = __vsub2(bq_cur, d);
+                base.x += (int) dlo;
+                base.y += (int) dhi;
+                if(st31) tab_out[t0 / kRebase] = base;
+            }
+            bq_nxt = load_above(t0 + 32);
+        }
+#pragma unroll
+        for(int u = 0; u < 8; ++u) {
+            W up = __shfl_up_sync(kFull, hlast, 1);
+            const uint32_t bv = __shfl_sync(kFull, bq_cur, (t0 & 31) + u);
+            if(lane == 0) up = bv;
+            if(!kG || (unsigned) j < (unsigned) ncols) {
+                const uint32_t *pb = prow + cur * SH;
+                W sc[4];
+                auto load_plane = [&](int q) {
+                    if(q < L::P16) {
+                        const uint4 v = *reinterpret_cast<const uint4 *>(pb + q * 128);
+                        sc[0] = v.x; sc[1] = v.y; sc[2] = v.z; sc[3] = v.w;
+                    } else {
+                        const uint2 v = *reinterpret_cast<const uint2 *>(pb + half_off);
+                        sc[0] = v.x; sc[1] = v.y;
+                    }
+                };
+                load_plane(0);
+                W above = up, dprev = diag;
+                uint4 pk;
+#pragma unroll
+                for(int r = 0; r < R; ++r) {
+                    W sr;
+                    if(r < L::R16) {
+                        if(r > 0 && (r & 3) == 0) load_plane(r >> 2);
+                        sr = sc[r & 3];
+                    } else {
+                        const int rr = r - L::R16;
+                        if((rr & 7) == 0) {
+                            if((rr >> 3) < L::P8) {
+                                pk = *reinterpret_cast<const uint4 *>(pb + L::PACK + (rr >> 3) * 128);
+                            } else {
+                                const uint2 v = *reinterpret_cast<const uint2 *>(pb + phalf_off);
+                                pk.x = v.x;
+                                pk.y = v.y;
+                            }
+                        }
+                        const int wi = (rr >> 1) & 3;
+                        const uint32_t w = wi == 0 ? pk.x : wi == 1 ? pk.y : wi == 2 ? pk.z : pk.w;
+                        sr = (rr & 1) ? prmt0<0x4341>(w) : prmt0<0x4240>(w);
+                    }
+                    const W Dg = __vadd2(dprev, sr);
+                    dprev = H[r];
+                    H[r] = __vimax3_u16x2(H[r], above, Dg);
+                    above = H[r];
+                }
+                hlast = H[R - 1];
+                if(st31) bound[j] = hlast;
+                diag = up;
+            }
+            cur = nxt;
+            nxt = cols[j + 2];
+            ++j;
+        }
+        // Columns 0 .. t0 + 7 - 31 of the last row are stored.
+        if(st31 && chain.mine && ((t0 + 8) & (kPublish - 1)) == 0 && t0 + 8 > 31)
+            st_release(chain.mine, (uint32_t) min(t0 + 8 - 31, ncols));
+    };
+
+    const int tend8 = (tend + 7) & ~7;
+    int t0 = 0;
+#pragma unroll 1
+    for(; t0 < tend8 && t0 < 32; t0 += 8) group(t0, Guard<true>{});
+#pragma unroll 1
+    for(; t0 + 7 < ncols; t0 += 8) group(t0, Guard<false>{});
+#pragma unroll 1
+    for(; t0 < tend8; t0 += 8) group(t0, Guard<true>{});
+    if(st31 && chain.mine) st_release(chain.mine, (uint32_t) ncols);
+}
+
 // The column sequences of one task: sorted b0, b0 + bstep, ... (ngrp of them
 // for this warp), each against the rows pair (x1, x2) of a job.
 struct TaskCols {
@@ -754,6 +964,50 @@ __device__ __noinline__ void narrow_task(uint32_t *sprof, const int8_t *g1, uint
         if(has && lane == 0) {
             jv.out[tri_index(tc.x1, y)] = r1;
             if(b != tc.a2) jv.out[tri_index(tc.x2, y)] = r2;
+        }
+    }
+}
+
+// Strips [s0, s1) of a 16-bit rows pair with strips of 32R rows on a moving
+// base, against one column sequence per warp: all of them, or one chained strip.
+template <int R, bool kPack>
+__device__ __noinline__ void long_task(uint32_t *sprof, const int8_t *g1, uint32_t lp1, const int8_t *g2, uint32_t lp2,
+                                       int e1, int e2, int s0, int s1, const TaskCols &tc, uint32_t *bound,
+                                       uint64_t words, const Chain &chain, uint32_t step, int32_t g, int lane)
+{
+    constexpr int SH = 32 * R;
+    const JobView &jv = *tc.jv;
+    const int slast = (e1 - 1) / SH, s2 = (e2 - 1) / SH;
+    const bool has = tc.b0 < jv.nclean;
+    const uint32_t y = has ? jv.sorted[tc.b0] : tc.x1;
+    const int ncols = has ? (int) jv.eff[y] : 0;
+    const uint8_t *cols = jv.units + jv.uoff[y];
+    const uint32_t entries = base_entries((uint32_t) ncols);
+    int2 *tabs = reinterpret_cast<int2 *>(bound + words) - kBaseTables * entries;
+    for(int s = s0; s < s1; ++s) {
+        const int i0 = s * SH;
+        __syncthreads();
+        stage_words<R, true, kPack>(sprof, g1, lp1, g2, lp2, i0, g);
+        __syncthreads();
+        if(!has) continue;
+        const bool last = s == slast;
+        const int k1 = last ? (e1 - 1 - i0) / R : 31;
+        Narrow::W H[R];
+        int2 base;
+        __syncwarp();
+        sweep_long<R, kPack>(sprof, cols, ncols, bound, tabs + (uint32_t) (s - 1) % kBaseTables * entries,
+                             tabs + (uint32_t) s % kBaseTables * entries, s == 0, ncols + k1, !last, chain, step, lane,
+                             H, base);
+        __syncwarp();
+        if(s == s2) {
+            const int rr = e2 - 1 - i0;
+            const int32_t v = __shfl_sync(kFull, base.y + Narrow::hi(pick_row<R, Narrow>(H, rr % R), g, e2, ncols), rr / R);
+            if(lane == 0 && tc.b0 != tc.a2) jv.out[tri_index(tc.x2, y)] = v;
+        }
+        if(last) {
+            const int rr = e1 - 1 - i0;
+            const int32_t v = __shfl_sync(kFull, base.x + Narrow::lo(pick_row<R, Narrow>(H, rr % R), g, e1, ncols), rr / R);
+            if(lane == 0) jv.out[tri_index(tc.x1, y)] = v;
         }
     }
 }
@@ -864,6 +1118,18 @@ __device__ __forceinline__ void strip_plan(int rows, int &nst, int &R)
 
 }  // namespace dev
 
+// Rows per lane of a rows pair's strips, from its flags: the plan's, or for a
+// chained one that would leave SMs idle, 16 or 8.
+template <int RMAX>
+__host__ __device__ __forceinline__ int strip_rows(int rows, uint8_t flags)
+{
+    if(flags & kRowR16) return 16;
+    if(flags & kRowR8) return 8;
+    const int nst = (rows + 32 * RMAX - 1) / (32 * RMAX);
+    const int R = (rows + 32 * nst - 1) / (32 * nst);
+    return (R + 1) & ~1;
+}
+
 // Resident CTAs per SM the batched kernel is compiled for (register budget).
 template <int RMAX, int W> struct BatchOcc { static constexpr int value = (RMAX == 32 ? 16 : 24) / W; };
 
@@ -881,7 +1147,9 @@ __host__ __device__ __forceinline__ uint32_t groups_per_task(uint32_t e1, int rm
 // All threads of the CTA call it.
 template <int RMAX, int W, bool kPack>
 __device__ __forceinline__ void rows_pair_task(const JobView &jv, uint32_t k, uint32_t grp, uint32_t ngrp,
-                                               uint32_t *sprof_b, uint32_t *bound, int warp, int lane)
+                                               uint32_t *sprof_b, uint32_t *bound, int warp, int lane,
+                                               uint64_t words = 0, uint32_t step = 0, int strip = -1,
+                                               const dev::Chain &chain = dev::Chain{nullptr, nullptr, nullptr})
 {
     const uint32_t a1 = 2 * k, a2 = min(2 * k + 1, jv.nclean - 1);
     const uint32_t x1 = jv.sorted[a1], x2 = jv.sorted[a2];
@@ -901,6 +1169,19 @@ __device__ __forceinline__ void rows_pair_task(const JobView &jv, uint32_t k, ui
                 MSA_QUAD(32) default: break;
             }
 #undef MSA_QUAD
+            return;
+        }
+        if(jv.row_narrow[k] & kRowLong) {
+            const int R = strip_rows<RMAX>(e1, jv.row_narrow[k]), nst = (e1 + 32 * R - 1) / (32 * R);
+            const int s0 = strip < 0 ? 0 : strip, s1 = strip < 0 ? nst : strip + 1;
+            const int8_t *g1 = jv.prof + jv.poff[x1], *g2 = jv.prof + jv.poff[x2];
+            const uint32_t lp1 = jv.plp[x1], lp2 = jv.plp[x2];
+#define MSA_LONG(RR) case RR: dev::long_task<RR, kPack>(sprof_b, g1, lp1, g2, lp2, e1, e2, s0, s1, tc, bound, words, chain, step, jv.g, lane); break;
+            switch(R) {   // strips of several per rows pair: 18 rows per lane and more, or 16 or 8
+                MSA_LONG(8) MSA_LONG(16) MSA_LONG(18) MSA_LONG(20) MSA_LONG(22) MSA_LONG(24) MSA_LONG(26) MSA_LONG(28)
+                MSA_LONG(30) MSA_LONG(32) default: break;
+            }
+#undef MSA_LONG
             return;
         }
     }
@@ -955,10 +1236,27 @@ __global__ void __launch_bounds__(W * 32, BatchOcc<RMAX, W>::value) nw_batched_k
             const uint32_t mid = (lo + hi + 1) >> 1;
             if(p.row_task[mid] <= q) lo = mid; else hi = mid - 1;
         }
+        if constexpr(RMAX == 32) {
+            const uint8_t fl = p.job.row_narrow[lo];
+            if(fl & kRowChain) {
+                // Task (group, strip); the strip above is the task before it.
+                const int e1 = (int) p.job.eff[p.job.sorted[2 * lo]], SH = 32 * strip_rows<RMAX>(e1, fl);
+                const uint32_t nst = (uint32_t) ((e1 + SH - 1) / SH), qq = (uint32_t) (q - p.row_task[lo]);
+                const uint32_t grp = qq / nst, strip = qq - grp * nst;
+                const uint64_t words = bound_words(p.job.eff[p.job.sorted[min(2 * lo + 1, p.job.nclean - 1)]]);
+                uint32_t *flag = p.chain_flag + task_q * W + warp;
+                const dev::Chain chain{strip ? flag - W : nullptr, flag, p.err};
+                rows_pair_task<RMAX, W, kPack>(p.job, lo, grp, 1, sprof_b,
+                                               p.chain_bound + p.chain_off[lo] + (grp * W + warp) * words, warp, lane,
+                                               words, p.step, (int) strip, chain);
+                continue;
+            }
+        }
         const uint32_t groups = (p.job.nclean - 2 * lo - 1 + W - 1) / W;
         const uint32_t chunk = groups_per_task(p.job.eff[p.job.sorted[2 * lo]], RMAX, p.gchunk);
         const uint32_t grp = (uint32_t) (q - p.row_task[lo]) * chunk;
-        rows_pair_task<RMAX, W, kPack>(p.job, lo, grp, min(chunk, groups - grp), sprof_b, bound, warp, lane);
+        rows_pair_task<RMAX, W, kPack>(p.job, lo, grp, min(chunk, groups - grp), sprof_b, bound, warp, lane,
+                                       p.bound_stride, p.step);
     }
 }
 
@@ -1084,6 +1382,17 @@ static inline bool narrow_ok(int64_t rows_p, int64_t cols, const ExtTable &t)
     return step * std::min(rows_p, cols) <= 0xffff;
 }
 
+// The largest s + 2g of the letters (and of padding rows, which score 0).
+static inline int64_t largest_step(const ExtTable &t) { return std::max<int64_t>(t.letter_pos, 0) + 2 * (int64_t) t.penalty; }
+
+// 16-bit lanes on a moving base are exact for any lengths when what lies
+// between the base and the largest cell in flight fits (sweep_long).
+static inline bool long_ok(const ExtTable &t)
+{
+    return (int64_t) t.letter_neg <= 2 * (int64_t) t.penalty && largest_step(t) <= 0xff &&
+           largest_step(t) * (32 * 32 + 34 + kRebase) <= 0xffff;
+}
+
 // Batched-kernel tile shapes (pick_tiles: rows per lane R and warps per CTA
 // W) and column groups per single-strip task (pick_chunk), autotuned; the
 // context may override either (msa_nw_set_tiles, msa_nw_set_variant).
@@ -1199,6 +1508,8 @@ struct NwPlan {
     uint32_t part = 0, nparts = 1;
     int variant = 0;            // msa_nw_set_variant flags the plan was built with
     uint32_t chunk = 0;         // and its groups-per-task override
+    size_t clear_bytes = 64;    // of the work counter and what follows it
+    bool chained = false;
     cudaGraphExec_t exec = nullptr;
     cudaStream_t captured_on = nullptr;
     ~NwPlan()
@@ -1213,6 +1524,8 @@ struct GraphCache {
 };
 
 static constexpr size_t kMaxPlans = 2;
+// Device memory that the boundary rows of chained rows pairs may take.
+static constexpr uint64_t kChainBytes = 2ull << 30;
 
 void release_graphs(msa_ctx *ctx)
 {
@@ -1299,7 +1612,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
 
     uint32_t max_cols = 1;
     for(uint32_t i = 0; i < n; ++i) max_cols = std::max(max_cols, st->plen[i]);
-    const uint64_t stride = round_up((uint64_t) max_cols + 160, 32);
+    const uint64_t stride = bound_words(max_cols);
 
     // Occupancy of the per-warp kernels.
     const size_t smem = smem_bytes<kPlainR>();
@@ -1313,13 +1626,15 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     // Persistent task tables: rows pairs (sorted 2k, 2k+1) x column groups of W.
     std::vector<uint64_t> row_task;
     std::vector<uint8_t> row_narrow;
+    std::vector<uint64_t> chain_off;
+    uint64_t chain_words = 0, chain_tasks = 0;
     uint64_t ntasks = 0;
     uint32_t K = 0;
     uint64_t task_base = 0;
     uint32_t gchunk = 1;
     if(mode == MSA_NW_PERSISTENT && nclean_pairs > 0) {
-        const int SH = 32 * tiles.R;
         K = (nclean + 1) / 2;
+        const int SH = 32 * tiles.R;
         row_narrow.assign(K, 0);
         std::vector<uint64_t> groups_k(K, 0);
         for(uint32_t k = 0; k < K; ++k) {
@@ -1329,6 +1644,8 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
             const int64_t cols = st->eff[st->clean_sorted[2 * k + 1]];
             const bool nar = narrow_ok(rows_p, cols, tbl) && !(ctx->nw_variant & MSA_NW_VARIANT_INT32);
             row_narrow[k] = nar ? kRowNarrow : 0;
+            if(!nar && tiles.R == 32 && long_ok(tbl) && !(ctx->nw_variant & MSA_NW_VARIANT_INT32))
+                row_narrow[k] = kRowNarrow | kRowLong;
             groups_k[k] = (uint64_t) (ncol + tiles.W - 1) / tiles.W;
             if(nar && k >= k_lo && k < k_hi) pl->narrow_tasks += (uint32_t) groups_k[k];
         }
@@ -1339,12 +1656,49 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
         // first's.
         if(tiles.R == 32 && narrow_ok(512, 512, tbl)) {
             for(uint32_t k = k_lo; k + 1 < k_hi; ++k) {
-                if(!(row_narrow[k] && row_narrow[k + 1])) continue;
+                if(row_narrow[k] != kRowNarrow || row_narrow[k + 1] != kRowNarrow) continue;
                 if(st->eff[st->clean_sorted[2 * k]] > 16 * 32) continue;
                 if(2 * (uint64_t) k + 3 >= nclean) break;
                 row_narrow[k] |= kRowQuad;
                 groups_k[k + 1] = 0;
                 ++k;
+            }
+        }
+        // Where the strips of the longest rows pair, one after the other, take
+        // more than the launch's share per resident CTA, it and those down to
+        // half of that share are chained: every strip a task, each waiting for
+        // the boundary row of the one above as it comes. (50 genomes: 4.7 ms,
+        // 5.4 when only those above the whole share are; where the longest is
+        // below it, the order of the tasks balances them, and chaining would
+        // cost 1,200 uneven sequences 0.3%.) Where the strips are too few for
+        // the CTAs, they are made lower.
+        chain_off.assign(K + 1, 0);
+        const uint64_t resident = 2 * (uint64_t) ctx->num_sms;
+        if(tiles.R == 32 && tiles.W == 8 && !ctx->nw_variant && !ctx->tile_r && long_ok(tbl)) {
+            auto eff_at = [&](uint32_t a) { return (uint64_t) st->eff[st->clean_sorted[std::min(a, nclean - 1)]]; };
+            // A task's time in instructions of one warp: steps times (rows per lane + 28).
+            auto task_cost = [&](uint32_t k) {
+                const uint64_t R = strip_rows<32>((int) eff_at(2 * k), 0), nst = (eff_at(2 * k) + 32 * R - 1) / (32 * R);
+                return nst * (eff_at(2 * k + 1) + 31) * (R + 28);
+            };
+            uint64_t total = 0;
+            for(uint32_t k = k_lo; k < k_hi; ++k) total += groups_k[k] * task_cost(k);
+            uint32_t kc = k_lo;
+            uint64_t strips = 0;
+            for(; kc < k_hi; ++kc) {
+                const uint64_t rows = eff_at(2 * kc), words = groups_k[kc] * 8 * bound_words((uint32_t) eff_at(2 * kc + 1));
+                if(rows <= 32 * 32 || !row_narrow[kc] || (kc == k_lo ? 1 : 2) * resident * task_cost(kc) < total) break;
+                if(chain_words + words > (kChainBytes >> 2)) break;
+                chain_off[kc] = chain_words;
+                chain_words += words;
+                strips += groups_k[kc] * ((rows + 1023) / 1024);
+            }
+            const uint8_t lower = strips >= resident ? 0 : 2 * strips >= resident ? kRowR16 : kRowR8;
+            for(uint32_t k = k_lo; k < kc; ++k) {
+                row_narrow[k] |= kRowLong | kRowChain | lower;
+                const uint64_t SH = 32 * (uint64_t) strip_rows<32>((int) eff_at(2 * k), row_narrow[k]);
+                groups_k[k] *= (eff_at(2 * k) + SH - 1) / SH;   // tasks
+                chain_tasks += groups_k[k];
             }
         }
         // Tasks of a single-strip rows pair take up to gchunk column groups
@@ -1382,7 +1736,10 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     auto take = [&off](size_t b) { size_t o = off; off = round_up(off + b, 256); return o; };
     const size_t o_prof = take(st->prof_bytes + 64), o_ext = take(kAlpha * kAlpha),
                  o_bound = take(warps_needed * stride * sizeof(uint32_t)), o_rt = take((K + 1) * sizeof(uint64_t)),
-                 o_rn = take(K + 16), o_gp = take(gpairs.size() * sizeof(uint32_t) + 16), o_cnt = take(64);
+                 o_rn = take(K + 16), o_co = take((K + 1) * sizeof(uint64_t)), o_cb = take(chain_words * sizeof(uint32_t)),
+                 o_gp = take(gpairs.size() * sizeof(uint32_t) + 16),
+                 // the work counter, the error word and the chained strips' progress, cleared by every launch
+                 o_cnt = take(64 + chain_tasks * 8 * sizeof(uint32_t));
     MSA_CUDA_TRY(ctx, pl->mem.ensure(off));
     char *base = (char *) pl->mem.ptr;
     cudaStream_t s = ctx->stream;
@@ -1390,6 +1747,8 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     if(K) {
         MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_rt, row_task.data(), (K + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
         MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_rn, row_narrow.data(), K, cudaMemcpyHostToDevice, s));
+        if(chain_tasks)
+            MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_co, chain_off.data(), (K + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
     }
     if(!gpairs.empty())
         MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_gp, gpairs.data(), gpairs.size() * sizeof(uint32_t),
@@ -1435,6 +1794,13 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     bp.bound = p.bound;
     bp.bound_stride = stride;
     bp.counter = (unsigned long long *) (base + o_cnt);
+    bp.err = (int *) (base + o_cnt + 8);
+    bp.chain_flag = (uint32_t *) (base + o_cnt + 64);
+    bp.chain_bound = (uint32_t *) (base + o_cb);
+    bp.chain_off = (const uint64_t *) (base + o_co);
+    bp.step = (uint32_t) std::min<int64_t>(largest_step(tbl), 0xffff);
+    pl->clear_bytes = 64 + chain_tasks * 8 * sizeof(uint32_t);
+    pl->chained = chain_tasks != 0;
 
     pl->launches = 1 + (pl->ngeneric ? 1 : 0);
     if(mode == MSA_NW_PLAIN && nclean_pairs > 0) {
@@ -1481,7 +1847,7 @@ static cudaError_t enqueue(msa_ctx *ctx, const NwPlan &pl, const SeqStore *st, c
             if((e = cudaGetLastError())) return e;
         }
     } else if(pl.bp.ntasks) {
-        if((e = cudaMemsetAsync(pl.bp.counter, 0, 64, s))) return e;
+        if((e = cudaMemsetAsync(pl.bp.counter, 0, pl.clear_bytes, s))) return e;
         const Tiles t = pl.tiles;
         if(pl.variant & MSA_NW_VARIANT_NO_PACKED) launch_batched<32, 8, false>(pl, s);
         else if(t.R == 16 && t.W == 4) launch_batched<16, 4>(pl, s);
@@ -1565,6 +1931,12 @@ int nw_run(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode, int32_t *d
     ctx->launches += pl->launches;
 
     MSA_CUDA_TRY(ctx, cudaEventSynchronize(ctx->ev[2]));
+    if(pl->chained) {
+        int err = 0;
+        MSA_CUDA_TRY(ctx, cudaMemcpyAsync(&err, pl->bp.err, sizeof(err), cudaMemcpyDeviceToHost, s));
+        MSA_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+        if(err) return set_error(ctx, MSA_ERR_DEVICE_TIMEOUT, "a wait between the strips of a sequence ran out");
+    }
     float ms_k = 0, ms_t = 0;
     cudaEventElapsedTime(&ms_k, ctx->ev[1], ctx->ev[2]);
     cudaEventElapsedTime(&ms_t, ctx->ev[0], ctx->ev[2]);

@@ -347,18 +347,19 @@ struct JobView {
     const uint64_t *poff;
     const uint32_t *plp;
     const uint32_t *sorted;     // clean sequences, eff descending
-    const uint8_t *row_narrow;  // per rows pair k: kRowNarrow, and kRowQuad for the first of a stacked pair
+    const uint8_t *row_narrow;  // per rows pair k: kRowNarrow and the flags beside it; for stacked ones on the first
     int32_t *out;
     uint32_t nclean;
     int32_t g;
 };
 
-// row_narrow flags: 16-bit lanes; rows pairs k and k + 1 stacked in one warp
-// (quad_task), their tasks all under k.
+// row_narrow flags: 16-bit lanes; rows pairs k and k + 1 (kRowQuad), or k to
+// k + 3 (kRowOct), stacked in one warp (stack_task), their tasks all under k.
 // Rows pairs of several strips: kRowLong runs its 16-bit lanes on a moving base
 // (sweep_long), kRowChain makes every strip a task of its own, of 32 x 32, 16 or
 // 8 rows (chain_rows).
-constexpr uint8_t kRowNarrow = 1, kRowQuad = 2, kRowLong = 4, kRowChain = 8, kRowR16 = 16, kRowR8 = 32;
+constexpr uint8_t kRowNarrow = 1, kRowQuad = 2, kRowLong = 4, kRowChain = 8, kRowR16 = 16, kRowR8 = 32,
+                  kRowOct = 64;
 
 // Steps between moves of a long strip's base; see sweep_long.
 constexpr int kRebase = 512;
@@ -456,15 +457,18 @@ __device__ __forceinline__ uint32_t prmt0(uint32_t w)
 // wholly inside or wholly past X2's profile.
 constexpr int kStageBatch = 4;
 
-// With msplit < 2R (16-bit lanes only), chunks m >= msplit (strip rows
-// 16 msplit and on) come from a second rows pair, (g1b, g2b) at their row
-// 16 (m - msplit): the stacked strip of quad_task.
-template <int R, bool kNarrow, bool kPack = true>
+// A rows pair's score profiles as staging reads them.
+struct RowsProf {
+    const int8_t *g1, *g2;
+    uint32_t lp1, lp2;
+};
+
+// With kPairs > 1 (16-bit lanes only) the strip stacks that many rows pairs,
+// each on 32 / kPairs lanes from its row 0: `stack` holds their profiles.
+template <int R, bool kNarrow, bool kPack = true, int kPairs = 1>
 __device__ __forceinline__ void stage_words(uint32_t *sprof, const int8_t *__restrict__ g1, uint32_t lp1,
                                             const int8_t *__restrict__ g2, uint32_t lp2, int i0, int32_t gap = 0,
-                                            const int8_t *__restrict__ g1b = nullptr, uint32_t lp1b = 0,
-                                            const int8_t *__restrict__ g2b = nullptr, uint32_t lp2b = 0,
-                                            int msplit = 1 << 30)
+                                            const RowsProf *stack = nullptr)
 {
     using L = Layout<R, kNarrow, kPack>;
     constexpr int SH = L::SH;
@@ -482,15 +486,16 @@ __device__ __forceinline__ void stage_words(uint32_t *sprof, const int8_t *__res
                 va[u] = vb[u] = make_uint4(0, 0, 0, 0);
                 if(c < TOTAL) {
                     const int b = c / CH, m = c - b * CH;
-                    if(m < msplit) {
+                    if constexpr(kPairs == 1) {
                         va[u] = __ldg(reinterpret_cast<const uint4 *>(g1 + (size_t) b * lp1 + i0) + m);
                         if((uint32_t) (i0 + 16 * m) < lp2)
                             vb[u] = __ldg(reinterpret_cast<const uint4 *>(g2 + (size_t) b * lp2 + i0) + m);
                     } else {
-                        const int mb = m - msplit;
-                        va[u] = __ldg(reinterpret_cast<const uint4 *>(g1b + (size_t) b * lp1b) + mb);
-                        if((uint32_t) (16 * mb) < lp2b)
-                            vb[u] = __ldg(reinterpret_cast<const uint4 *>(g2b + (size_t) b * lp2b) + mb);
+                        constexpr int CPP = CH / kPairs;   // chunks per rows pair
+                        const RowsProf &rp = stack[m / CPP];
+                        const int mb = m % CPP;
+                        va[u] = __ldg(reinterpret_cast<const uint4 *>(rp.g1 + (size_t) b * rp.lp1) + mb);
+                        vb[u] = __ldg(reinterpret_cast<const uint4 *>(rp.g2 + (size_t) b * rp.lp2) + mb);
                     }
                 }
             }
@@ -569,8 +574,8 @@ template <bool V> struct Guard { static constexpr bool value = V; };
 //              back when store_bound);
 //   kTopZero   row zero of the gap-free state, 0, above lane 0 (a strip that
 //              is the first and the last one, 16-bit lanes only);
-//   kTopStack  as kTopZero, and lanes 16..31 hold a second rows pair of its
-//              own whose row zero sits above lane 16 (see quad_task).
+//   kTopStack  as kTopZero, with a rows pair of its own on every LP lanes, row
+//              zero above the first of them (see stack_task).
 constexpr int kTopBound = 0, kTopZero = 1, kTopStack = 2;
 
 // Sweeps one strip (rows [i0, i0 + 32R)) of one column sequence on the calling
@@ -579,8 +584,9 @@ constexpr int kTopBound = 0, kTopZero = 1, kTopStack = 2;
 // H registers hold the strip's rows at the last column it reached
 // (tend - 1 - lane). Steps run in groups of 8 (the loop bookkeeping of a group
 // is shared by 8 columns); only the fill and drain groups, where some lanes
-// sit outside [0, ncols), test the lane's column.
-template <int R, class K, bool kPack = true, int kTop = kTopBound>
+// sit outside [0, ncols), test the lane's column. Lane k is one step behind lane
+// k - 1 of its rows pair.
+template <int R, class K, bool kPack = true, int kTop = kTopBound, int LP = 32>
 __device__ __forceinline__ void sweep_strip(const uint32_t *__restrict__ sprof, const uint8_t *__restrict__ cols,
                                             int ncols, uint32_t *__restrict__ bound, int i0, int tend,
                                             bool store_bound, int32_t g, int lane, typename K::W (&H)[R])
@@ -611,7 +617,7 @@ __device__ __forceinline__ void sweep_strip(const uint32_t *__restrict__ sprof, 
     const int half_off = L::HALF - lane * 2;      // the 16-bit half plane, from prow
     const int phalf_off = L::PHALF - lane * 2;    // the packed half plane, from prow
     const bool st31 = store_bound && lane == 31;
-    int j = -lane;
+    int j = -(lane & (LP - 1));
     uint32_t cur = cols[j], nxt = cols[j + 1];   // columns -32..ncols+35 lie in the padded store
 
     auto group = [&](int t0, auto guard) {
@@ -629,7 +635,7 @@ __device__ __forceinline__ void sweep_strip(const uint32_t *__restrict__ sprof, 
             } else if constexpr(kTop == kTopZero) {
                 if(lane == 0) up = 0u;
             } else {
-                if((lane & 15) == 0) up = 0u;
+                if((lane & (LP - 1)) == 0) up = 0u;
             }
             if(!kG || (unsigned) j < (unsigned) ncols) {
                 const uint32_t *pb = prow + cur * SH;
@@ -706,7 +712,7 @@ __device__ __forceinline__ void sweep_strip(const uint32_t *__restrict__ sprof, 
     const int tend4 = (tend + 7) & ~7;
     int t0 = 0;
 #pragma unroll 1
-    for(; t0 < tend4 && t0 < 32; t0 += 8) group(t0, Guard<true>{});
+    for(; t0 < tend4 && t0 < LP; t0 += 8) group(t0, Guard<true>{});
 #pragma unroll 1
     for(; t0 + 7 < ncols; t0 += 8) group(t0, Guard<false>{});   // every lane inside [0, ncols)
 #pragma unroll 1
@@ -1054,55 +1060,45 @@ __device__ __noinline__ void wide_task(uint32_t *sprof, const int8_t *g1, uint32
     }
 }
 
-// Two short rows pairs in one warp: pair A (sorted 2k, 2k+1) on lanes 0..15
-// and pair B (sorted 2k+2, 2k+3) on lanes 16..31, R rows per lane, so each
-// pair has 16R >= its rows in one strip; both sweep the same column
-// sequences (those of pair A: sorted 2k+1 + q W + warp). In the gap-free
-// state row zero is 0, so lane 16 takes 0 from above instead of lane 15's
-// last row, and the two halves never mix. A column is scored for a rows
-// sequence only when it comes after it in the sorted order. Halves the
-// per-step overhead per cell against a 16R-row strip on 32 lanes.
-template <int R, bool kPack>
-__device__ __noinline__ void quad_task(uint32_t *sprof, const JobView &jv, uint32_t k, uint32_t b0, uint32_t bstep,
-                                       uint32_t ngrp, int32_t g, int lane)
+// kPairs short rows pairs (2 or 4) in one warp: pair k + p (sorted 2(k + p),
+// 2(k + p) + 1) on LP = 32 / kPairs lanes from p LP on, R rows per lane, so each
+// pair has LP R >= its rows in one strip; all sweep the same column sequences
+// (those of pair k: sorted 2k + 1 + q W + warp). In the gap-free state row zero
+// is 0, so the first lane of a pair takes 0 from above instead of the last row
+// of the pair before, and they never mix. A column is scored for a rows sequence
+// only when it comes after it in the sorted order; the lane that holds a
+// sequence's last row writes its score. A step's fixed cost (about 28
+// instructions) is shared by kPairs times the cells of a strip on 32 lanes, and
+// filling and draining the lanes takes LP - 1 steps per column sequence instead
+// of 31: 3,000 reads of 100 to 250 bases 13.9 -> 9.06 ms (two by two before).
+template <int R, int kPairs, bool kPack>
+__device__ __noinline__ void stack_task(uint32_t *sprof, RowsProf *stack, const JobView &jv, uint32_t k, uint32_t b0,
+                                        uint32_t bstep, uint32_t ngrp, int32_t g, int lane)
 {
-    const uint32_t xa1 = jv.sorted[2 * k], xa2 = jv.sorted[2 * k + 1];
-    const uint32_t xb1 = jv.sorted[2 * k + 2], xb2 = jv.sorted[2 * k + 3];
-    const int ea1 = (int) jv.eff[xa1], ea2 = (int) jv.eff[xa2], eb1 = (int) jv.eff[xb1], eb2 = (int) jv.eff[xb2];
+    constexpr int LP = 32 / kPairs;
+    if(threadIdx.x < kPairs) {   // read after the barrier below; the last task's stagings are over
+        const uint32_t s1 = jv.sorted[2 * (k + threadIdx.x)], s2 = jv.sorted[2 * (k + threadIdx.x) + 1];
+        stack[threadIdx.x] = RowsProf{jv.prof + jv.poff[s1], jv.prof + jv.poff[s2], jv.plp[s1], jv.plp[s2]};
+    }
+    __syncthreads();
+    stage_words<R, true, kPack, kPairs>(sprof, nullptr, 0, nullptr, 0, 0, g, stack);
+    __syncthreads();
+    // The lane's rows pair, and whether it holds the last row of either sequence.
+    const uint32_t a1 = 2 * (k + lane / LP), x1 = jv.sorted[a1], x2 = jv.sorted[a1 + 1];
+    const int l1 = (int) jv.eff[x1] - 1, l2 = (int) jv.eff[x2] - 1, at = lane % LP;
     for(uint32_t t = 0; t < ngrp; ++t) {
         const uint32_t b = b0 + t * bstep;
-        const bool has = b < jv.nclean;
-        const uint32_t y = has ? jv.sorted[b] : xa1;
-        const int ncols = has ? (int) jv.eff[y] : 0;
-        const uint8_t *cols = jv.units + jv.uoff[y];
-        if(t == 0) {
-            __syncthreads();
-            stage_words<R, true, kPack>(sprof, jv.prof + jv.poff[xa1], jv.plp[xa1], jv.prof + jv.poff[xa2],
-                                        jv.plp[xa2], 0, g, jv.prof + jv.poff[xb1], jv.plp[xb1],
-                                        jv.prof + jv.poff[xb2], jv.plp[xb2], R);
-            __syncthreads();
-        }
-        if(has) {
-            Narrow::W H[R];
-            __syncwarp();
-            // Lane 31 is the last one to reach a column (pair B's rows).
-            sweep_strip<R, Narrow, kPack, kTopStack>(sprof, cols, ncols, nullptr, 0, ncols + 31, false, g, lane, H);
-            __syncwarp();
-            auto take = [&](int rows, int lane0, bool hi) {
-                const int rr = rows - 1;
-                const Narrow::W w = pick_row<R, Narrow>(H, rr % R);
-                const int32_t v = hi ? Narrow::hi(w, g, rows, ncols) : Narrow::lo(w, g, rows, ncols);
-                return __shfl_sync(kFull, v, lane0 + rr / R);
-            };
-            const int32_t ra1 = take(ea1, 0, false), ra2 = take(ea2, 0, true);
-            const int32_t rb1 = take(eb1, 16, false), rb2 = take(eb2, 16, true);
-            if(lane == 0) {
-                jv.out[tri_index(xa1, y)] = ra1;
-                if(b > 2 * k + 1) jv.out[tri_index(xa2, y)] = ra2;
-                if(b > 2 * k + 2) jv.out[tri_index(xb1, y)] = rb1;
-                if(b > 2 * k + 3) jv.out[tri_index(xb2, y)] = rb2;
-            }
-        }
+        if(b >= jv.nclean) break;
+        const uint32_t y = jv.sorted[b];
+        const int ncols = (int) jv.eff[y];
+        Narrow::W H[R];
+        __syncwarp();
+        sweep_strip<R, Narrow, kPack, kTopStack, LP>(sprof, jv.units + jv.uoff[y], ncols, nullptr, 0, ncols + LP - 1,
+                                                     false, g, lane, H);
+        __syncwarp();
+        const Narrow::W w1 = pick_row<R, Narrow>(H, l1 % R), w2 = pick_row<R, Narrow>(H, l2 % R);
+        if(at == l1 / R && b > a1) jv.out[tri_index(x1, y)] = Narrow::lo(w1, g, l1 + 1, ncols);
+        if(at == l2 / R && b > a1 + 1) jv.out[tri_index(x2, y)] = Narrow::hi(w2, g, l2 + 1, ncols);
     }
 }
 
@@ -1157,20 +1153,30 @@ __device__ __forceinline__ void rows_pair_task(const JobView &jv, uint32_t k, ui
     dev::TaskCols tc{&jv, x1, x2, a2, 2 * k + 1 + grp * W + warp, (uint32_t) W, ngrp};
 
     if constexpr(RMAX == 32) {
+        __shared__ dev::RowsProf stack[4];
+        // Stacked rows pairs: R rows per lane, enough for pair k's longer first
+        // sequence.
+#define MSA_STACK(RR, NP) case RR: dev::stack_task<RR, NP, kPack>(sprof_b, stack, jv, k, tc.b0, tc.bstep, ngrp, jv.g, lane); break;
+#define MSA_STACKS(NP)                                                                                              \
+    switch(R) {                                                                                                     \
+        MSA_STACK(2, NP) MSA_STACK(4, NP) MSA_STACK(6, NP) MSA_STACK(8, NP) MSA_STACK(10, NP) MSA_STACK(12, NP)     \
+        MSA_STACK(14, NP) MSA_STACK(16, NP) MSA_STACK(18, NP) MSA_STACK(20, NP) MSA_STACK(22, NP) MSA_STACK(24, NP) \
+        MSA_STACK(26, NP) MSA_STACK(28, NP) MSA_STACK(30, NP) MSA_STACK(32, NP) default: break;                     \
+    }
         if(jv.row_narrow[k] & kRowQuad) {
-            // Rows pairs k and k + 1 stacked (quad_task): R rows per lane, 16R
-            // covering pair k's longer first sequence.
-            int R = (e1 + 15) / 16;
-            R = (R + 1) & ~1;
-#define MSA_QUAD(RR) case RR: dev::quad_task<RR, kPack>(sprof_b, jv, k, tc.b0, tc.bstep, ngrp, jv.g, lane); break;
-            switch(R) {
-                MSA_QUAD(2) MSA_QUAD(4) MSA_QUAD(6) MSA_QUAD(8) MSA_QUAD(10) MSA_QUAD(12) MSA_QUAD(14) MSA_QUAD(16)
-                MSA_QUAD(18) MSA_QUAD(20) MSA_QUAD(22) MSA_QUAD(24) MSA_QUAD(26) MSA_QUAD(28) MSA_QUAD(30)
-                MSA_QUAD(32) default: break;
-            }
-#undef MSA_QUAD
+            const int R = ((e1 + 15) / 16 + 1) & ~1;
+            MSA_STACKS(2)
             return;
         }
+        if constexpr(kPack) {
+            if(jv.row_narrow[k] & kRowOct) {
+                const int R = ((e1 + 7) / 8 + 1) & ~1;
+                MSA_STACKS(4)
+                return;
+            }
+        }
+#undef MSA_STACKS
+#undef MSA_STACK
         if(jv.row_narrow[k] & kRowLong) {
             const int R = strip_rows<RMAX>(e1, jv.row_narrow[k]), nst = (e1 + 32 * R - 1) / (32 * R);
             const int s0 = strip < 0 ? 0 : strip, s1 = strip < 0 ? nst : strip + 1;
@@ -1649,20 +1655,34 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
             groups_k[k] = (uint64_t) (ncol + tiles.W - 1) / tiles.W;
             if(nar && k >= k_lo && k < k_hi) pl->narrow_tasks += (uint32_t) groups_k[k];
         }
-        // Short rows pairs two by two in one warp (quad_task): both on 16-bit
-        // lanes with the state bound holding for 512 rows, the first's
-        // longer sequence within 16 x 32 rows, the second with two sequences
-        // and columns, and both in this part. The second's tasks are the
-        // first's.
+        // Short rows pairs stacked in one warp (stack_task), four by four up to
+        // 256 rows and two by two up to 512: all on 16-bit lanes with the state
+        // bound holding for 512 rows, the first's longer sequence within the
+        // lanes, the last with two sequences and columns, and all in this
+        // part. The others' tasks are the first's. Stacking leaves fewer tasks,
+        // so it is used where at least two per resident CTA are left (120
+        // proteins of 80 to 600 residues: 172 us stacked two by two, 143 us not;
+        // 257 of 150 to 400: 274 us stacked, 350 us not).
         if(tiles.R == 32 && narrow_ok(512, 512, tbl)) {
-            for(uint32_t k = k_lo; k + 1 < k_hi; ++k) {
-                if(row_narrow[k] != kRowNarrow || row_narrow[k + 1] != kRowNarrow) continue;
-                if(st->eff[st->clean_sorted[2 * k]] > 16 * 32) continue;
-                if(2 * (uint64_t) k + 3 >= nclean) break;
-                row_narrow[k] |= kRowQuad;
-                groups_k[k + 1] = 0;
-                ++k;
-            }
+            uint64_t groups_all = 0;
+            for(uint32_t k = k_lo; k < k_hi; ++k) groups_all += groups_k[k];
+            const uint64_t fill = 4 * (uint64_t) ctx->num_sms;   // twice the resident CTAs
+            auto stack = [&](uint32_t pairs, uint32_t rows, uint8_t flag) {
+                if(groups_all < pairs * fill) return;
+                for(uint32_t k = k_lo; k + pairs <= k_hi;) {
+                    bool ok = st->eff[st->clean_sorted[2 * k]] <= rows && 2 * ((uint64_t) k + pairs) <= nclean;
+                    for(uint32_t p = 0; p < pairs; ++p) ok = ok && row_narrow[k + p] == kRowNarrow && groups_k[k + p] != 0;
+                    if(!ok) {
+                        ++k;
+                        continue;
+                    }
+                    row_narrow[k] |= flag;
+                    for(uint32_t p = 1; p < pairs; ++p) groups_k[k + p] = 0;
+                    k += pairs;
+                }
+            };
+            if(tiles.W == 8 && !(ctx->nw_variant & MSA_NW_VARIANT_NO_PACKED)) stack(4, 8 * 32, kRowOct);
+            stack(2, 16 * 32, kRowQuad);
         }
         // Where the strips of the longest rows pair, one after the other, take
         // more than the launch's share per resident CTA, it and those down to

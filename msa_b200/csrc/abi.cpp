@@ -170,8 +170,8 @@ int build_store(msa_ctx *ctx, const uint8_t *units, const uint64_t *offs, const 
             scan_units(src, st->len[i], st->plen[i], &st->eff[i], &st->dirty[i], &st->has_gap[i]);
             st->any_gap |= st->has_gap[i] != 0;
         }
-        // Clean sequences sorted by effective length, longest first.
-        sort_clean(st->eff, st->dirty, st->clean_sorted);
+        st->end_dirty = st->dirty;
+        order_clean(st->eff, st->len, st->any_gap, st->dirty, st->clean_sorted);
         // Profile geometry.
         st->prof_off.resize(n);
         st->prof_lp.resize(n);
@@ -318,9 +318,8 @@ static int all_pairs(msa_ctx *ctx, msa_seqs seqs, const msa_table *table, int mo
         const uint64_t npairs = (uint64_t) st->n * (st->n ? st->n - 1 : 0) / 2;
         if(npairs && !out) return MSA_ERR_INVALID;
         // Tables that are not symmetric make the score depend on orientation:
-        // route every pair through the reference-orientation path for this
-        // call. The store's own plan comes back on every exit, exceptions
-        // included.
+        // the clean sequences are put into the reference's for this call. The
+        // store's own order comes back on every exit, exceptions included.
         struct Reorient {
             SeqStore *st;
             bool active;
@@ -331,8 +330,8 @@ static int all_pairs(msa_ctx *ctx, msa_seqs seqs, const msa_table *table, int mo
                 if(!active) return;
                 dirty = st->dirty;
                 sorted = st->clean_sorted;
-                std::fill(st->dirty.begin(), st->dirty.end(), 1);
-                st->clean_sorted.clear();
+                st->dirty = st->end_dirty;
+                order_clean(st->eff, st->len, true, st->dirty, st->clean_sorted);
             }
             ~Reorient()
             {

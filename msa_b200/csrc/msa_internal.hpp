@@ -54,7 +54,8 @@ struct SeqStore {
     std::vector<uint64_t> len;      // given length (units)
     std::vector<uint32_t> eff;      // index of first END unit within the padded length
     std::vector<uint32_t> plen;     // 3 * ceil(len / 3)
-    std::vector<uint8_t> dirty;     // END units not forming a suffix, or eff == 0
+    std::vector<uint8_t> dirty;     // scored by the generic kernel (order_clean)
+    std::vector<uint8_t> end_dirty; // END units not forming a suffix, or eff == 0
     std::vector<uint8_t> has_gap;   // a GAP unit within the padded length
     std::vector<uint64_t> off;      // byte offset of the units in d_units
     uint8_t *d_units = nullptr;
@@ -63,7 +64,7 @@ struct SeqStore {
     uint32_t *d_eff = nullptr;
     uint32_t *d_plen = nullptr;
     bool any_gap = false;
-    // Clean sequences sorted by eff descending (ties: original index ascending).
+    // Clean sequences, longest first (order_clean).
     std::vector<uint32_t> clean_sorted;
     uint32_t *d_clean_sorted = nullptr;
     // Profile geometry per sequence (original index): Lp = round_up(max(eff,1), kProfPad).
@@ -131,10 +132,17 @@ int nw_run(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode, int32_t *d
 
 // Host-side sequence scan (the rules of a store upload): index of the first
 // END unit within the padded length, "dirty" (END units not forming a
-// suffix, empty, or a GAP unit) and GAP presence.
+// suffix, or empty) and GAP presence.
 void scan_units(const uint8_t *src, uint64_t len, uint32_t plen, uint32_t *eff, uint8_t *dirty, uint8_t *gap);
-// Clean sequences sorted by eff descending (ties: index ascending).
-void sort_clean(const std::vector<uint32_t> &eff, const std::vector<uint8_t> &dirty, std::vector<uint32_t> &out);
+// The clean sequences in the order in which the batched and plain kernels take
+// the earlier one of a pair as its rows. Where a score does not depend on the
+// orientation: by eff descending (ties: index ascending). Where it does (a GAP
+// unit anywhere, a table that is not symmetric; `oriented`): the reference's
+// orientation, rows = more 3-unit blocks, ties to the smaller index, as one
+// order; sequences whose END suffix holds whole blocks become dirty then,
+// because their length does not follow from their blocks.
+void order_clean(const std::vector<uint32_t> &eff, const std::vector<uint64_t> &len, bool oriented,
+                 std::vector<uint8_t> &dirty, std::vector<uint32_t> &out);
 // Pairs with at least one dirty sequence, row-major, each as (rows, columns)
 // in the reference's orientation.
 void list_generic_pairs(const std::vector<uint8_t> &dirty, const std::vector<uint64_t> &len,

@@ -379,6 +379,9 @@ __host__ __device__ __forceinline__ uint64_t bound_words(uint32_t ncols)
 {
     return ((uint64_t) ncols + 160 + 2 * kBaseTables * base_entries(ncols) + 31) / 32 * 32;
 }
+// The same for the columns of a rows pair, its second sequence and those after
+// it in the sorted order, which may be longer by the rest of a 3-unit block.
+__host__ __device__ __forceinline__ uint64_t chain_words_of(uint32_t second) { return bound_words((second + 2) / 3 * 3); }
 
 struct BatchParams {
     JobView job;
@@ -929,7 +932,7 @@ __device__ __noinline__ void narrow_task(uint32_t *sprof, const int8_t *g1, uint
 {
     constexpr int SH = 32 * R;
     const JobView &jv = *tc.jv;
-    const int s2 = (e2 - 1) / SH;
+    const int em = max(e1, e2), s1 = (e1 - 1) / SH, s2 = (e2 - 1) / SH;
     for(uint32_t t = 0; t < tc.ngrp; ++t) {
         const uint32_t b = tc.b0 + t * tc.bstep;
         const bool has = b < jv.nclean;
@@ -949,7 +952,7 @@ __device__ __noinline__ void narrow_task(uint32_t *sprof, const int8_t *g1, uint
             }
             if(has) {
                 const bool last = s == nst - 1;
-                const int k1 = last ? (e1 - 1 - i0) / R : 31;
+                const int k1 = last ? (em - 1 - i0) / R : 31;
                 Narrow::W H[R];
                 __syncwarp();
                 if(nst == 1)
@@ -961,7 +964,7 @@ __device__ __noinline__ void narrow_task(uint32_t *sprof, const int8_t *g1, uint
                     const int rr = e2 - 1 - i0;
                     r2 = __shfl_sync(kFull, Narrow::hi(pick_row<R, Narrow>(H, rr % R), g, e2, ncols), rr / R);
                 }
-                if(last) {
+                if(s == s1) {
                     const int rr = e1 - 1 - i0;
                     r1 = __shfl_sync(kFull, Narrow::lo(pick_row<R, Narrow>(H, rr % R), g, e1, ncols), rr / R);
                 }
@@ -983,7 +986,7 @@ __device__ __noinline__ void long_task(uint32_t *sprof, const int8_t *g1, uint32
 {
     constexpr int SH = 32 * R;
     const JobView &jv = *tc.jv;
-    const int slast = (e1 - 1) / SH, s2 = (e2 - 1) / SH;
+    const int em = max(e1, e2), slast = (em - 1) / SH, sr1 = (e1 - 1) / SH, sr2 = (e2 - 1) / SH;
     const bool has = tc.b0 < jv.nclean;
     const uint32_t y = has ? jv.sorted[tc.b0] : tc.x1;
     const int ncols = has ? (int) jv.eff[y] : 0;
@@ -997,7 +1000,7 @@ __device__ __noinline__ void long_task(uint32_t *sprof, const int8_t *g1, uint32
         __syncthreads();
         if(!has) continue;
         const bool last = s == slast;
-        const int k1 = last ? (e1 - 1 - i0) / R : 31;
+        const int k1 = last ? (em - 1 - i0) / R : 31;
         Narrow::W H[R];
         int2 base;
         __syncwarp();
@@ -1005,12 +1008,12 @@ __device__ __noinline__ void long_task(uint32_t *sprof, const int8_t *g1, uint32
                              tabs + (uint32_t) s % kBaseTables * entries, s == 0, ncols + k1, !last, chain, step, lane,
                              H, base);
         __syncwarp();
-        if(s == s2) {
+        if(s == sr2) {
             const int rr = e2 - 1 - i0;
             const int32_t v = __shfl_sync(kFull, base.y + Narrow::hi(pick_row<R, Narrow>(H, rr % R), g, e2, ncols), rr / R);
             if(lane == 0 && tc.b0 != tc.a2) jv.out[tri_index(tc.x2, y)] = v;
         }
-        if(last) {
+        if(s == sr1) {
             const int rr = e1 - 1 - i0;
             const int32_t v = __shfl_sync(kFull, base.x + Narrow::lo(pick_row<R, Narrow>(H, rr % R), g, e1, ncols), rr / R);
             if(lane == 0) jv.out[tri_index(tc.x1, y)] = v;
@@ -1149,13 +1152,18 @@ __device__ __forceinline__ void rows_pair_task(const JobView &jv, uint32_t k, ui
 {
     const uint32_t a1 = 2 * k, a2 = min(2 * k + 1, jv.nclean - 1);
     const uint32_t x1 = jv.sorted[a1], x2 = jv.sorted[a2];
-    const int e1 = (int) jv.eff[x1], e2 = (int) jv.eff[x2];
+    // In the reference's orientation the second may be up to two rows longer.
+    const int e1 = (int) jv.eff[x1], e2 = (int) jv.eff[x2], em = max(e1, e2);
     dev::TaskCols tc{&jv, x1, x2, a2, 2 * k + 1 + grp * W + warp, (uint32_t) W, ngrp};
 
     if constexpr(RMAX == 32) {
         __shared__ dev::RowsProf stack[4];
-        // Stacked rows pairs: R rows per lane, enough for pair k's longer first
-        // sequence.
+        // Stacked rows pairs: R rows per lane, enough for the longest sequence.
+        auto longest = [&](uint32_t pairs) {
+            int e = em;
+            for(uint32_t a = 2 * k + 2; a < 2 * (k + pairs); ++a) e = max(e, (int) jv.eff[jv.sorted[a]]);
+            return e;
+        };
 #define MSA_STACK(RR, NP) case RR: dev::stack_task<RR, NP, kPack>(sprof_b, stack, jv, k, tc.b0, tc.bstep, ngrp, jv.g, lane); break;
 #define MSA_STACKS(NP)                                                                                              \
     switch(R) {                                                                                                     \
@@ -1164,13 +1172,13 @@ __device__ __forceinline__ void rows_pair_task(const JobView &jv, uint32_t k, ui
         MSA_STACK(26, NP) MSA_STACK(28, NP) MSA_STACK(30, NP) MSA_STACK(32, NP) default: break;                     \
     }
         if(jv.row_narrow[k] & kRowQuad) {
-            const int R = ((e1 + 15) / 16 + 1) & ~1;
+            const int R = ((longest(2) + 15) / 16 + 1) & ~1;
             MSA_STACKS(2)
             return;
         }
         if constexpr(kPack) {
             if(jv.row_narrow[k] & kRowOct) {
-                const int R = ((e1 + 7) / 8 + 1) & ~1;
+                const int R = ((longest(4) + 7) / 8 + 1) & ~1;
                 MSA_STACKS(4)
                 return;
             }
@@ -1178,7 +1186,7 @@ __device__ __forceinline__ void rows_pair_task(const JobView &jv, uint32_t k, ui
 #undef MSA_STACKS
 #undef MSA_STACK
         if(jv.row_narrow[k] & kRowLong) {
-            const int R = strip_rows<RMAX>(e1, jv.row_narrow[k]), nst = (e1 + 32 * R - 1) / (32 * R);
+            const int R = strip_rows<RMAX>(em, jv.row_narrow[k]), nst = (em + 32 * R - 1) / (32 * R);
             const int s0 = strip < 0 ? 0 : strip, s1 = strip < 0 ? nst : strip + 1;
             const int8_t *g1 = jv.prof + jv.poff[x1], *g2 = jv.prof + jv.poff[x2];
             const uint32_t lp1 = jv.plp[x1], lp2 = jv.plp[x2];
@@ -1193,7 +1201,7 @@ __device__ __forceinline__ void rows_pair_task(const JobView &jv, uint32_t k, ui
     }
     if(jv.row_narrow[k]) {
         int nst, R;
-        dev::strip_plan<RMAX>(e1, nst, R);
+        dev::strip_plan<RMAX>(em, nst, R);
         const int8_t *g1 = jv.prof + jv.poff[x1], *g2 = jv.prof + jv.poff[x2];
         const uint32_t lp1 = jv.plp[x1], lp2 = jv.plp[x2];
 #define MSA_NARROW(RR) case RR: dev::narrow_task<RR, kPack>(sprof_b, g1, lp1, g2, lp2, e1, e2, nst, tc, bound, jv.g, lane); break;
@@ -1246,10 +1254,11 @@ __global__ void __launch_bounds__(W * 32, BatchOcc<RMAX, W>::value) nw_batched_k
             const uint8_t fl = p.job.row_narrow[lo];
             if(fl & kRowChain) {
                 // Task (group, strip); the strip above is the task before it.
-                const int e1 = (int) p.job.eff[p.job.sorted[2 * lo]], SH = 32 * strip_rows<RMAX>(e1, fl);
-                const uint32_t nst = (uint32_t) ((e1 + SH - 1) / SH), qq = (uint32_t) (q - p.row_task[lo]);
+                const uint32_t second = p.job.eff[p.job.sorted[min(2 * lo + 1, p.job.nclean - 1)]];
+                const int em = (int) max(p.job.eff[p.job.sorted[2 * lo]], second), SH = 32 * strip_rows<RMAX>(em, fl);
+                const uint32_t nst = (uint32_t) ((em + SH - 1) / SH), qq = (uint32_t) (q - p.row_task[lo]);
                 const uint32_t grp = qq / nst, strip = qq - grp * nst;
-                const uint64_t words = bound_words(p.job.eff[p.job.sorted[min(2 * lo + 1, p.job.nclean - 1)]]);
+                const uint64_t words = chain_words_of(second);
                 uint32_t *flag = p.chain_flag + task_q * W + warp;
                 const dev::Chain chain{strip ? flag - W : nullptr, flag, p.err};
                 rows_pair_task<RMAX, W, kPack>(p.job, lo, grp, 1, sprof_b,
@@ -1259,7 +1268,9 @@ __global__ void __launch_bounds__(W * 32, BatchOcc<RMAX, W>::value) nw_batched_k
             }
         }
         const uint32_t groups = (p.job.nclean - 2 * lo - 1 + W - 1) / W;
-        const uint32_t chunk = groups_per_task(p.job.eff[p.job.sorted[2 * lo]], RMAX, p.gchunk);
+        const uint32_t chunk = groups_per_task(max(p.job.eff[p.job.sorted[2 * lo]],
+                                                   p.job.eff[p.job.sorted[min(2 * lo + 1, p.job.nclean - 1)]]),
+                                               RMAX, p.gchunk);
         const uint32_t grp = (uint32_t) (q - p.row_task[lo]) * chunk;
         rows_pair_task<RMAX, W, kPack>(p.job, lo, grp, min(chunk, groups - grp), sprof_b, bound, warp, lane,
                                        p.bound_stride, p.step);
@@ -1377,26 +1388,36 @@ static int occupancy(KernelT kernel, size_t smem, int *blocks)
 // its matched cells, so with smin + 2g >= 0 the state and its diagonal
 // candidate lie in [0, min(i,j)*(smax + 2g)], with min(i,j) <= min(rows, cols).
 // Cells outside the sequences (padding rows, the shorter sequence's tail) may
-// wrap within their half but never feed a scored cell. Clean sequences hold
-// letter units only, so smin and smax are taken over the letter block.
-static inline bool narrow_ok(int64_t rows_p, int64_t cols, const ExtTable &t)
+// wrap within their half but never feed a scored cell. smin and smax are taken
+// over the letter block, or, where sequences hold GAP units, over every entry
+// but END's.
+struct ScoreRange { int64_t pos, neg; };   // largest score, largest magnitude of a negative one
+static inline ScoreRange range_of(const ExtTable &t, bool gap)
 {
+    return gap ? ScoreRange{t.max_pos, t.max_neg} : ScoreRange{t.letter_pos, t.letter_neg};
+}
+static inline bool narrow_ok(int64_t rows_p, int64_t cols, const ExtTable &t, bool gap = false)
+{
+    const ScoreRange sr = range_of(t, gap);
     const int64_t g2 = 2 * (int64_t) t.penalty;
-    if((int64_t) t.letter_neg > g2) return false;
-    const int64_t step = std::max<int64_t>((int64_t) t.letter_pos + g2, 0);
+    if(sr.neg > g2) return false;
+    const int64_t step = std::max<int64_t>(sr.pos + g2, 0);
     if(step > 0xff) return false;   // s + 2g is staged as a byte in packed rows
     return step * std::min(rows_p, cols) <= 0xffff;
 }
 
 // The largest s + 2g of the letters (and of padding rows, which score 0).
-static inline int64_t largest_step(const ExtTable &t) { return std::max<int64_t>(t.letter_pos, 0) + 2 * (int64_t) t.penalty; }
+static inline int64_t largest_step(const ExtTable &t, bool gap)
+{
+    return std::max<int64_t>(range_of(t, gap).pos, 0) + 2 * (int64_t) t.penalty;
+}
 
 // 16-bit lanes on a moving base are exact for any lengths when what lies
 // between the base and the largest cell in flight fits (sweep_long).
-static inline bool long_ok(const ExtTable &t)
+static inline bool long_ok(const ExtTable &t, bool gap)
 {
-    return (int64_t) t.letter_neg <= 2 * (int64_t) t.penalty && largest_step(t) <= 0xff &&
-           largest_step(t) * (32 * 32 + 34 + kRebase) <= 0xffff;
+    return range_of(t, gap).neg <= 2 * (int64_t) t.penalty && largest_step(t, gap) <= 0xff &&
+           largest_step(t, gap) * (32 * 32 + 34 + kRebase) <= 0xffff;
 }
 
 // Batched-kernel tile shapes (pick_tiles: rows per lane R and warps per CTA
@@ -1641,16 +1662,19 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     if(mode == MSA_NW_PERSISTENT && nclean_pairs > 0) {
         K = (nclean + 1) / 2;
         const int SH = 32 * tiles.R;
+        const bool gap = st->any_gap;
+        auto eff_at = [&](uint32_t a) { return (uint64_t) st->eff[st->clean_sorted[std::min(a, nclean - 1)]]; };
+        // Rows of rows pair k, and its longest column sequence.
+        auto rows_at = [&](uint32_t k) { return std::max(eff_at(2 * k), eff_at(2 * k + 1)); };
+        auto cols_at = [&](uint32_t k) { return gap || !table_is_symmetric(tbl) ? (eff_at(2 * k + 1) + 2) / 3 * 3 : eff_at(2 * k + 1); };
         row_narrow.assign(K, 0);
         std::vector<uint64_t> groups_k(K, 0);
         for(uint32_t k = 0; k < K; ++k) {
             const int64_t ncol = (int64_t) nclean - (2 * (int64_t) k + 1);
             if(ncol <= 0) continue;
-            const int64_t rows_p = (int64_t) round_up(st->eff[st->clean_sorted[2 * k]], SH);
-            const int64_t cols = st->eff[st->clean_sorted[2 * k + 1]];
-            const bool nar = narrow_ok(rows_p, cols, tbl) && !(ctx->nw_variant & MSA_NW_VARIANT_INT32);
+            const bool nar = narrow_ok((int64_t) round_up(rows_at(k), SH), (int64_t) cols_at(k), tbl, gap) && !(ctx->nw_variant & MSA_NW_VARIANT_INT32);
             row_narrow[k] = nar ? kRowNarrow : 0;
-            if(!nar && tiles.R == 32 && long_ok(tbl) && !(ctx->nw_variant & MSA_NW_VARIANT_INT32))
+            if(!nar && tiles.R == 32 && long_ok(tbl, gap) && !(ctx->nw_variant & MSA_NW_VARIANT_INT32))
                 row_narrow[k] = kRowNarrow | kRowLong;
             groups_k[k] = (uint64_t) (ncol + tiles.W - 1) / tiles.W;
             if(nar && k >= k_lo && k < k_hi) pl->narrow_tasks += (uint32_t) groups_k[k];
@@ -1663,15 +1687,16 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
         // so it is used where at least two per resident CTA are left (120
         // proteins of 80 to 600 residues: 172 us stacked two by two, 143 us not;
         // 257 of 150 to 400: 274 us stacked, 350 us not).
-        if(tiles.R == 32 && narrow_ok(512, 512, tbl)) {
+        if(tiles.R == 32 && narrow_ok(512, 512, tbl, gap)) {
             uint64_t groups_all = 0;
             for(uint32_t k = k_lo; k < k_hi; ++k) groups_all += groups_k[k];
             const uint64_t fill = 4 * (uint64_t) ctx->num_sms;   // twice the resident CTAs
             auto stack = [&](uint32_t pairs, uint32_t rows, uint8_t flag) {
                 if(groups_all < pairs * fill) return;
                 for(uint32_t k = k_lo; k + pairs <= k_hi;) {
-                    bool ok = st->eff[st->clean_sorted[2 * k]] <= rows && 2 * ((uint64_t) k + pairs) <= nclean;
-                    for(uint32_t p = 0; p < pairs; ++p) ok = ok && row_narrow[k + p] == kRowNarrow && groups_k[k + p] != 0;
+                    bool ok = 2 * ((uint64_t) k + pairs) <= nclean;
+                    for(uint32_t p = 0; p < pairs; ++p)
+                        ok = ok && row_narrow[k + p] == kRowNarrow && groups_k[k + p] != 0 && rows_at(k + p) <= rows;
                     if(!ok) {
                         ++k;
                         continue;
@@ -1694,19 +1719,18 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
         // the CTAs, they are made lower.
         chain_off.assign(K + 1, 0);
         const uint64_t resident = 2 * (uint64_t) ctx->num_sms;
-        if(tiles.R == 32 && tiles.W == 8 && !ctx->nw_variant && !ctx->tile_r && long_ok(tbl)) {
-            auto eff_at = [&](uint32_t a) { return (uint64_t) st->eff[st->clean_sorted[std::min(a, nclean - 1)]]; };
+        if(tiles.R == 32 && tiles.W == 8 && !ctx->nw_variant && !ctx->tile_r && long_ok(tbl, gap)) {
             // A task's time in instructions of one warp: steps times (rows per lane + 28).
             auto task_cost = [&](uint32_t k) {
-                const uint64_t R = strip_rows<32>((int) eff_at(2 * k), 0), nst = (eff_at(2 * k) + 32 * R - 1) / (32 * R);
-                return nst * (eff_at(2 * k + 1) + 31) * (R + 28);
+                const uint64_t R = strip_rows<32>((int) rows_at(k), 0), nst = (rows_at(k) + 32 * R - 1) / (32 * R);
+                return nst * (cols_at(k) + 31) * (R + 28);
             };
             uint64_t total = 0;
             for(uint32_t k = k_lo; k < k_hi; ++k) total += groups_k[k] * task_cost(k);
             uint32_t kc = k_lo;
             uint64_t strips = 0;
             for(; kc < k_hi; ++kc) {
-                const uint64_t rows = eff_at(2 * kc), words = groups_k[kc] * 8 * bound_words((uint32_t) eff_at(2 * kc + 1));
+                const uint64_t rows = rows_at(kc), words = groups_k[kc] * 8 * chain_words_of((uint32_t) eff_at(2 * kc + 1));
                 if(rows <= 32 * 32 || !row_narrow[kc] || (kc == k_lo ? 1 : 2) * resident * task_cost(kc) < total) break;
                 if(chain_words + words > (kChainBytes >> 2)) break;
                 chain_off[kc] = chain_words;
@@ -1716,8 +1740,8 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
             const uint8_t lower = strips >= resident ? 0 : 2 * strips >= resident ? kRowR16 : kRowR8;
             for(uint32_t k = k_lo; k < kc; ++k) {
                 row_narrow[k] |= kRowLong | kRowChain | lower;
-                const uint64_t SH = 32 * (uint64_t) strip_rows<32>((int) eff_at(2 * k), row_narrow[k]);
-                groups_k[k] *= (eff_at(2 * k) + SH - 1) / SH;   // tasks
+                const uint64_t SH = 32 * (uint64_t) strip_rows<32>((int) rows_at(k), row_narrow[k]);
+                groups_k[k] *= (rows_at(k) + SH - 1) / SH;   // tasks
                 chain_tasks += groups_k[k];
             }
         }
@@ -1729,7 +1753,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
             uint64_t nt = 0;
             for(uint32_t k = 0; k < K; ++k) {
                 row_task[k] = nt;
-                const uint32_t c = groups_per_task(st->eff[st->clean_sorted[2 * k]], tiles.R, chunk);
+                const uint32_t c = groups_per_task((uint32_t) rows_at(k), tiles.R, chunk);
                 nt += (groups_k[k] + c - 1) / c;
             }
             row_task[K] = nt;
@@ -1757,7 +1781,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     const size_t o_prof = take(st->prof_bytes + 64), o_ext = take(kAlpha * kAlpha),
                  o_bound = take(warps_needed * stride * sizeof(uint32_t)), o_rt = take((K + 1) * sizeof(uint64_t)),
                  o_rn = take(K + 16), o_co = take((K + 1) * sizeof(uint64_t)), o_cb = take(chain_words * sizeof(uint32_t)),
-                 o_gp = take(gpairs.size() * sizeof(uint32_t) + 16),
+                 o_gp = take(gpairs.size() * sizeof(uint32_t) + 16), o_ord = take(nclean * sizeof(uint32_t) + 16),
                  // the work counter, the error word and the chained strips' progress, cleared by every launch
                  o_cnt = take(64 + chain_tasks * 8 * sizeof(uint32_t));
     MSA_CUDA_TRY(ctx, pl->mem.ensure(off));
@@ -1770,6 +1794,9 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
         if(chain_tasks)
             MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_co, chain_off.data(), (K + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
     }
+    if(nclean)
+        MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_ord, st->clean_sorted.data(), nclean * sizeof(uint32_t),
+                                          cudaMemcpyHostToDevice, s));
     if(!gpairs.empty())
         MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_gp, gpairs.data(), gpairs.size() * sizeof(uint32_t),
                                           cudaMemcpyHostToDevice, s));
@@ -1784,7 +1811,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     p.prof = (const int8_t *) (base + o_prof);
     p.poff = st->d_prof_off;
     p.plp = st->d_prof_lp;
-    p.sorted = st->d_clean_sorted;
+    p.sorted = (const uint32_t *) (base + o_ord);   // the call's order, not always the store's
     p.nclean = nclean;
     p.out = d_out;
     p.g = tbl.penalty;
@@ -1801,7 +1828,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     bp.job.prof = p.prof;
     bp.job.poff = st->d_prof_off;
     bp.job.plp = st->d_prof_lp;
-    bp.job.sorted = st->d_clean_sorted;
+    bp.job.sorted = p.sorted;
     bp.job.nclean = nclean;
     bp.job.row_narrow = (const uint8_t *) (base + o_rn);
     bp.job.out = d_out;
@@ -1818,7 +1845,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     bp.chain_flag = (uint32_t *) (base + o_cnt + 64);
     bp.chain_bound = (uint32_t *) (base + o_cb);
     bp.chain_off = (const uint64_t *) (base + o_co);
-    bp.step = (uint32_t) std::min<int64_t>(largest_step(tbl), 0xffff);
+    bp.step = (uint32_t) std::min<int64_t>(largest_step(tbl, st->any_gap), 0xffff);
     pl->clear_bytes = 64 + chain_tasks * 8 * sizeof(uint32_t);
     pl->chained = chain_tasks != 0;
 

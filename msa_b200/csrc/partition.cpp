@@ -34,15 +34,21 @@ void scan_units(const uint8_t *src, uint64_t len, uint32_t plen, uint32_t *eff, 
     if(!seen_end && len < plen) first_end = (uint32_t) len;
     *eff = first_end;
     *gap = g ? 1 : 0;
-    *dirty = (d || first_end == 0 || g) ? 1 : 0;
+    *dirty = (d || first_end == 0) ? 1 : 0;
 }
 
-void sort_clean(const std::vector<uint32_t> &eff, const std::vector<uint8_t> &dirty, std::vector<uint32_t> &out)
+void order_clean(const std::vector<uint32_t> &eff, const std::vector<uint64_t> &len, bool oriented,
+                 std::vector<uint8_t> &dirty, std::vector<uint32_t> &out)
 {
     out.clear();
-    for(uint32_t i = 0; i < (uint32_t) eff.size(); ++i)
+    for(uint32_t i = 0; i < (uint32_t) eff.size(); ++i) {
+        if(oriented && (eff[i] + 2) / 3 != (len[i] + 2) / 3) dirty[i] = 1;
         if(!dirty[i]) out.push_back(i);
-    std::stable_sort(out.begin(), out.end(), [&eff](uint32_t a, uint32_t b) { return eff[a] > eff[b]; });
+    }
+    if(oriented)
+        std::stable_sort(out.begin(), out.end(), [&len](uint32_t a, uint32_t b) { return (len[a] + 2) / 3 > (len[b] + 2) / 3; });
+    else
+        std::stable_sort(out.begin(), out.end(), [&eff](uint32_t a, uint32_t b) { return eff[a] > eff[b]; });
 }
 
 void list_generic_pairs(const std::vector<uint8_t> &dirty, const std::vector<uint64_t> &len,
@@ -135,9 +141,9 @@ extern "C" int msa_nw_part_of_pairs(const uint8_t *units, const uint64_t *offs, 
             plen[i] = (uint32_t) ((lens[i] + 2) / 3 * 3);
             scan_units(units + offs[i], lens[i], plen[i], &eff[i], &dirty[i], &gap[i]);
         }
-        if(!table_is_symmetric(ext)) std::fill(dirty.begin(), dirty.end(), 1);
+        const bool any_gap = std::find(gap.begin(), gap.end(), 1) != gap.end();
         std::vector<uint32_t> sorted, gpairs;
-        sort_clean(eff, dirty, sorted);
+        order_clean(eff, len, any_gap || !table_is_symmetric(ext), dirty, sorted);
         list_generic_pairs(dirty, len, gpairs);
         const JobSplit s = split_job(eff, plen, sorted, gpairs, nparts);
         auto tri = [](uint64_t i, uint64_t j) { return i > j ? i * (i - 1) / 2 + j : j * (j - 1) / 2 + i; };

@@ -141,7 +141,7 @@ static uint64_t task_cells(const Job *j, uint32_t k, uint32_t g)
 
 // Whether a job needs the reference's orientation (the single-job path):
 // a sequence with END units before its last letter, an empty one or one with
-// GAP units (the store's "dirty" rule, scan_units), a table that is not
+// GAP units (scan_units), a table that is not
 // symmetric, or fewer than two sequences. Decided on the host from the job's
 // units.
 bool needs_reference_orientation(const Job *j)
@@ -155,7 +155,7 @@ bool needs_reference_orientation(const Job *j)
         uint32_t eff = 0;
         uint8_t dirty = 0, gap = 0;
         scan_units(j->units.data() + j->offs[i], j->lens[i], plen, &eff, &dirty, &gap);
-        if(dirty) return true;
+        if(dirty || gap) return true;
     }
     return false;
 }
@@ -187,8 +187,8 @@ int score_oriented(msa_server *srv, Job *j)
         for(int y = 0; y < 25; ++y)
             if(j->ext.score[x * kAlpha + y] != j->ext.score[y * kAlpha + x]) { symmetric = false; break; }
     if(!symmetric) {
-        std::fill(st->dirty.begin(), st->dirty.end(), 1);
-        st->clean_sorted.clear();
+        st->dirty = st->end_dirty;
+        order_clean(st->eff, st->len, true, st->dirty, st->clean_sorted);
     }
     void *out = nullptr;
     cudaError_t e = cudaMallocFromPoolAsync(&out, npairs * 4, srv->pool, ctx->stream);

@@ -30,6 +30,62 @@ void DevBuf::release()
     bytes = 0;
 }
 
+cudaError_t BlockCache::take(size_t need, void **ptr, size_t *bytes)
+{
+    size_t want = std::max<size_t>(need, 4096), unit = 1024;
+    while(unit * 8 < want) unit *= 2;
+    want = round_up(want, unit);   // unit is between an eighth and a quarter of it
+    for(size_t k = m_free.size(); k-- > 0;)
+        if(m_free[k].bytes == want) {
+            *ptr = m_free[k].ptr;
+            *bytes = want;
+            m_total -= want;
+            m_free.erase(m_free.begin() + k);
+            return cudaSuccess;
+        }
+    cudaError_t e = cudaMalloc(ptr, want);
+    if(e != cudaSuccess && !m_free.empty()) {
+        cudaGetLastError();
+        clear();
+        e = cudaMalloc(ptr, want);
+    }
+    if(e != cudaSuccess) {
+        cudaGetLastError();
+        *ptr = nullptr;
+        return e;
+    }
+    *bytes = want;
+    return cudaSuccess;
+}
+
+void BlockCache::give(void *ptr, size_t bytes)
+{
+    if(!ptr) return;
+    if(bytes > kCacheBytes / 2) {
+        cudaFree(ptr);
+        return;
+    }
+    try {
+        m_free.push_back({ptr, bytes});
+    } catch(...) {
+        cudaFree(ptr);
+        return;
+    }
+    m_total += bytes;
+    while(m_total > kCacheBytes || m_free.size() > kCacheBlocks) {
+        cudaFree(m_free.front().ptr);
+        m_total -= m_free.front().bytes;
+        m_free.erase(m_free.begin());
+    }
+}
+
+void BlockCache::clear()
+{
+    for(const Block &b : m_free) cudaFree(b.ptr);
+    m_free.clear();
+    m_total = 0;
+}
+
 int set_error(msa_ctx *ctx, int status, const std::string &msg)
 {
     if(ctx) ctx->err = msg;
@@ -46,11 +102,9 @@ int cuda_error(msa_ctx *ctx, cudaError_t e, const char *what)
 static void free_store(SeqStore *st)
 {
     if(!st) return;
-    void *bufs[] = {st->d_units, st->d_off, st->d_eff, st->d_plen, st->d_clean_sorted, st->d_prof_off, st->d_prof_lp};
-    for(void *p : bufs) {
-        if(!p) continue;
-        if(st->pooled) cudaFreeAsync(p, st->free_stream);
-        else cudaFree(p);
+    if(st->block) {
+        if(st->pooled) cudaFreeAsync(st->block, st->free_stream);
+        else st->home->blocks.give(st->block, st->block_bytes);
     }
     delete st;
 }
@@ -108,6 +162,7 @@ void msa_destroy(msa_ctx *ctx)
     ctx->out_tmp.release();
     ctx->pairs.release();
     ctx->nj_buf.release();
+    ctx->blocks.clear();
     for(auto &e : ctx->ev) if(e) cudaEventDestroy(e);
     if(ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
@@ -158,15 +213,22 @@ int build_store(msa_ctx *ctx, const uint8_t *units, const uint64_t *offs, const 
             total += round_up(st->plen[i] + kUnitPad, 16);
         }
         st->units_bytes = total + kUnitPad;
-        std::vector<uint8_t> host(st->units_bytes, (uint8_t) MSA_UNIT_END);
+        // One device block and one copy: the units, then the arrays that say
+        // where they are, each 16-byte aligned.
+        size_t at = round_up(st->units_bytes, 16);
+        auto take = [&at](size_t b) { const size_t o = at; at = round_up(at + b, 16); return o; };
+        const size_t o_off = take(n * sizeof(uint64_t)), o_eff = take(n * sizeof(uint32_t)),
+                     o_plen = take(n * sizeof(uint32_t)), o_sorted = take(n * sizeof(uint32_t)),
+                     o_poff = take(n * sizeof(uint64_t)), o_plp = take(n * sizeof(uint32_t));
+        std::vector<uint8_t> host(at, (uint8_t) MSA_UNIT_END);
         for(uint32_t i = 0; i < n; ++i) {
             const uint8_t *src = units + offs[i];
             uint8_t *dst = host.data() + st->off[i];
-            for(uint64_t k = 0; k < st->len[i]; ++k) {
-                const uint8_t u = src[k];
-                if(u > MSA_UNIT_GAP) { free_store(st); return set_error(ctx, MSA_ERR_INVALID, "unit code above 25"); }
-                dst[k] = u;
+            if(unit_kinds(src, st->len[i]) & 4) {
+                free_store(st);
+                return set_error(ctx, MSA_ERR_INVALID, "unit code above 25");
             }
+            if(st->len[i]) std::memcpy(dst, src, st->len[i]);
             scan_units(src, st->len[i], st->plen[i], &st->eff[i], &st->dirty[i], &st->has_gap[i]);
             st->any_gap |= st->has_gap[i] != 0;
         }
@@ -183,30 +245,32 @@ int build_store(msa_ctx *ctx, const uint8_t *units, const uint64_t *offs, const 
         }
         st->prof_bytes = poff;
 
+        auto put = [&](size_t o, const void *src, size_t b) { if(b) std::memcpy(host.data() + o, src, b); };
+        put(o_off, st->off.data(), n * sizeof(uint64_t));
+        put(o_eff, st->eff.data(), n * sizeof(uint32_t));
+        put(o_plen, st->plen.data(), n * sizeof(uint32_t));
+        put(o_sorted, st->clean_sorted.data(), st->clean_sorted.size() * sizeof(uint32_t));
+        put(o_poff, st->prof_off.data(), n * sizeof(uint64_t));
+        put(o_plp, st->prof_lp.data(), n * sizeof(uint32_t));
+
         st->pooled = ctx->pool != nullptr;
         st->free_stream = ctx->stream;
-        auto dmalloc = [&](void **p, size_t b) {
-            return st->pooled ? cudaMallocFromPoolAsync(p, std::max<size_t>(b, 16), ctx->pool, ctx->stream)
-                              : cudaMalloc(p, std::max<size_t>(b, 16));
-        };
-        cudaError_t e = cudaSuccess;
-        if(!e) e = dmalloc((void **) &st->d_units, st->units_bytes);
-        if(!e) e = dmalloc((void **) &st->d_off, n * sizeof(uint64_t));
-        if(!e) e = dmalloc((void **) &st->d_eff, n * sizeof(uint32_t));
-        if(!e) e = dmalloc((void **) &st->d_plen, n * sizeof(uint32_t));
-        if(!e) e = dmalloc((void **) &st->d_clean_sorted, st->clean_sorted.size() * sizeof(uint32_t));
-        if(!e) e = dmalloc((void **) &st->d_prof_off, n * sizeof(uint64_t));
-        if(!e) e = dmalloc((void **) &st->d_prof_lp, n * sizeof(uint32_t));
+        st->home = ctx;
         cudaStream_t s = ctx->stream;
-        if(!e) e = cudaMemcpyAsync(st->d_units, host.data(), st->units_bytes, cudaMemcpyHostToDevice, s);
-        if(!e && n) e = cudaMemcpyAsync(st->d_off, st->off.data(), n * sizeof(uint64_t), cudaMemcpyHostToDevice, s);
-        if(!e && n) e = cudaMemcpyAsync(st->d_eff, st->eff.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice, s);
-        if(!e && n) e = cudaMemcpyAsync(st->d_plen, st->plen.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice, s);
-        if(!e && !st->clean_sorted.empty())
-            e = cudaMemcpyAsync(st->d_clean_sorted, st->clean_sorted.data(), st->clean_sorted.size() * sizeof(uint32_t),
-                                cudaMemcpyHostToDevice, s);
-        if(!e && n) e = cudaMemcpyAsync(st->d_prof_off, st->prof_off.data(), n * sizeof(uint64_t), cudaMemcpyHostToDevice, s);
-        if(!e && n) e = cudaMemcpyAsync(st->d_prof_lp, st->prof_lp.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice, s);
+        cudaError_t e = st->pooled ? cudaMallocFromPoolAsync(&st->block, at, ctx->pool, s)
+                                   : ctx->blocks.take(at, &st->block, &st->block_bytes);
+        if(e) st->block = nullptr;
+        if(!e) {
+            uint8_t *base = (uint8_t *) st->block;
+            st->d_units = base;
+            st->d_off = (uint64_t *) (base + o_off);
+            st->d_eff = (uint32_t *) (base + o_eff);
+            st->d_plen = (uint32_t *) (base + o_plen);
+            st->d_clean_sorted = (uint32_t *) (base + o_sorted);
+            st->d_prof_off = (uint64_t *) (base + o_poff);
+            st->d_prof_lp = (uint32_t *) (base + o_plp);
+            e = cudaMemcpyAsync(base, host.data(), at, cudaMemcpyHostToDevice, s);
+        }
         if(!e) e = cudaStreamSynchronize(s);   // host staging buffer goes out of scope
         if(e) { free_store(st); return cuda_error(ctx, e, "sequence upload"); }
         static std::atomic<uint64_t> serials{1};

@@ -11,6 +11,8 @@
 
 #include <cuda_runtime.h>
 
+struct msa_ctx;
+
 #include "../../include/msa_b200.h"
 
 namespace msa {
@@ -58,6 +60,8 @@ struct SeqStore {
     std::vector<uint8_t> end_dirty; // END units not forming a suffix, or eff == 0
     std::vector<uint8_t> has_gap;   // a GAP unit within the padded length
     std::vector<uint64_t> off;      // byte offset of the units in d_units
+    void *block = nullptr;          // the device allocation that holds every d_ array
+    size_t block_bytes = 0;
     uint8_t *d_units = nullptr;
     uint64_t units_bytes = 0;
     uint64_t *d_off = nullptr;
@@ -74,9 +78,10 @@ struct SeqStore {
     uint64_t *d_prof_off = nullptr;
     uint32_t *d_prof_lp = nullptr;
     std::vector<std::string> names;   // record descriptions (msa_seqs_load_fasta)
-    // Device buffers came from the context's memory pool in stream order; they
-    // are returned in stream order on free_stream.
+    // The block came from the context's memory pool in stream order and is
+    // returned in stream order on free_stream; else it goes back to `home`.
     bool pooled = false;
+    msa_ctx *home = nullptr;
     cudaStream_t free_stream = nullptr;
 };
 
@@ -88,12 +93,35 @@ struct DevBuf {
     void release();
 };
 
+// Device blocks of released stores and plans, kept for the next ones: a
+// cudaMalloc and cudaFree pair costs from 10 us to milliseconds, as much as a
+// small call. Sizes are rounded up to quarters of a power of two so that
+// similar calls share them. Used by the context's thread only, and only for
+// blocks that no work in flight touches. Holds at most kCacheBytes in
+// kCacheBlocks blocks; emptied when an allocation fails and with the context.
+class BlockCache {
+public:
+    cudaError_t take(size_t need, void **ptr, size_t *bytes);
+    void give(void *ptr, size_t bytes);
+    void clear();
+
+private:
+    static constexpr size_t kCacheBytes = size_t(1) << 30;
+    static constexpr size_t kCacheBlocks = 16;
+    struct Block { void *ptr; size_t bytes; };
+    std::vector<Block> m_free;   // oldest first
+    size_t m_total = 0;
+};
+
 struct GraphCache;
 
 }  // namespace msa
 
 struct msa_ctx {
     int device = 0;
+    msa::BlockCache blocks;
+    int plain_blocks_per_sm = 0;      // of the per-warp kernels, once asked for
+    int batch_blocks_per_sm[5] = {};  // of the batched kernel's instances
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     std::string err;
@@ -130,6 +158,8 @@ struct NwPlan;
 int nw_run(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode, int32_t *d_out, uint32_t part = 0,
            uint32_t nparts = 1);
 
+// What a run of units holds: bit 0 END units, bit 1 GAP units, bit 2 codes above 25.
+uint8_t unit_kinds(const uint8_t *src, uint64_t len);
 // Host-side sequence scan (the rules of a store upload): index of the first
 // END unit within the padded length, "dirty" (END units not forming a
 // suffix, or empty) and GAP presence.

@@ -1522,7 +1522,10 @@ struct NwPlan {
     int32_t *d_out = nullptr;
     Tiles tiles{0, 0};
     ExtTable tbl{};
-    DevBuf mem;
+    msa_ctx *home = nullptr;    // whose block cache `mem` goes back to
+    void *mem = nullptr;
+    size_t mem_bytes = 0;
+    std::vector<uint8_t> staged;   // host copy of the tables at the start of `mem`
     const int8_t *d_ext = nullptr;
     NwParams p{};
     BatchParams bp{};
@@ -1542,15 +1545,45 @@ struct NwPlan {
     ~NwPlan()
     {
         if(exec) cudaGraphExecDestroy(exec);
-        mem.release();
+        if(mem) home->blocks.give(mem, mem_bytes);
     }
 };
 
 struct GraphCache {
     std::vector<NwPlan *> plans;   // most recent last
+    // Executable graphs of dropped plans: a new plan's sequence mostly has the
+    // same nodes, and updating one costs a fraction of instantiating it.
+    std::vector<cudaGraphExec_t> spare;
+    void drop(NwPlan *pl)
+    {
+        if(pl->exec && spare.size() < 4) {
+            spare.push_back(pl->exec);
+            pl->exec = nullptr;
+        }
+        delete pl;
+    }
+    // `g` as an executable graph.
+    cudaError_t instantiate(cudaGraph_t g, cudaGraphExec_t *exec)
+    {
+        while(!spare.empty()) {
+            cudaGraphExec_t x = spare.back();
+            spare.pop_back();
+            cudaGraphExecUpdateResultInfo info{};
+            if(cudaGraphExecUpdate(x, g, &info) == cudaSuccess) {
+                *exec = x;
+                return cudaSuccess;
+            }
+            cudaGetLastError();
+            cudaGraphExecDestroy(x);
+        }
+        return cudaGraphInstantiate(exec, g, 0);
+    }
 };
 
-static constexpr size_t kMaxPlans = 2;
+// Plans kept per context: as many as a program rotates its stores through, and
+// at most kMaxPlanBytes beyond the newest.
+static constexpr size_t kMaxPlans = 8;
+static constexpr size_t kMaxPlanBytes = size_t(2) << 30;
 // Device memory that the boundary rows of chained rows pairs may take.
 static constexpr uint64_t kChainBytes = 2ull << 30;
 
@@ -1558,6 +1591,7 @@ void release_graphs(msa_ctx *ctx)
 {
     if(!ctx->graphs) return;
     for(NwPlan *pl : ctx->graphs->plans) delete pl;
+    for(cudaGraphExec_t x : ctx->graphs->spare) cudaGraphExecDestroy(x);
     delete ctx->graphs;
     ctx->graphs = nullptr;
 }
@@ -1567,20 +1601,26 @@ void drop_plans_for_store(msa_ctx *ctx, uint64_t serial)
     if(!ctx->graphs) return;
     auto &v = ctx->graphs->plans;
     for(size_t i = 0; i < v.size();) {
-        if(v[i]->store_serial == serial) { delete v[i]; v.erase(v.begin() + i); }
+        if(v[i]->store_serial == serial) { ctx->graphs->drop(v[i]); v.erase(v.begin() + i); }
         else ++i;
     }
 }
 
+// Grid of an instance of the batched kernel (`slot`: its place in the context's
+// occupancy cache).
 template <int R, int W, bool kPack = true>
-static int batched_grid(msa_ctx *ctx, uint64_t ntasks, uint64_t *grid)
+static int batched_grid(msa_ctx *ctx, int slot, uint64_t ntasks, uint64_t *grid)
 {
-    auto kern = nw_batched_kernel<R, W, kPack>;
-    const size_t smem = (size_t) kAlpha * 32 * R * 4;
-    MSA_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-    int bps = 0;
-    MSA_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, W * 32, smem));
-    if(bps < 1) return set_error(ctx, MSA_ERR_CUDA, "batched NW kernel cannot be resident");
+    int &bps = ctx->batch_blocks_per_sm[slot];
+    if(bps == 0) {
+        auto kern = nw_batched_kernel<R, W, kPack>;
+        const size_t smem = (size_t) kAlpha * 32 * R * 4;
+        MSA_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+        int k = 0;
+        MSA_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kern, W * 32, smem));
+        if(k < 1) return set_error(ctx, MSA_ERR_CUDA, "batched NW kernel cannot be resident");
+        bps = k;
+    }
     *grid = std::min<uint64_t>((uint64_t) ctx->num_sms * bps, std::max<uint64_t>(ntasks, 1));
     return MSA_OK;
 }
@@ -1641,13 +1681,18 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     for(uint32_t i = 0; i < n; ++i) max_cols = std::max(max_cols, st->plen[i]);
     const uint64_t stride = bound_words(max_cols);
 
-    // Occupancy of the per-warp kernels.
-    const size_t smem = smem_bytes<kPlainR>();
-    int bps = 0, bps3 = 0;
-    if(occupancy(nw_plain_kernel<kPlainR, kWPB>, smem, &bps) || occupancy(nw_generic_kernel<kPlainR, kWPB>, smem, &bps3))
-        return set_error(ctx, MSA_ERR_CUDA, "occupancy query failed (no sm_100a image?)");
-    bps = std::min(bps, bps3);
-    const uint64_t resident_blocks = (uint64_t) ctx->num_sms * (uint64_t) bps;
+    // Occupancy of the per-warp kernels, where they run.
+    uint64_t resident_blocks = 0;
+    if(mode == MSA_NW_PLAIN || pl->ngeneric) {
+        if(ctx->plain_blocks_per_sm == 0) {
+            const size_t smem = smem_bytes<kPlainR>();
+            int bps = 0, bps3 = 0;
+            if(occupancy(nw_plain_kernel<kPlainR, kWPB>, smem, &bps) || occupancy(nw_generic_kernel<kPlainR, kWPB>, smem, &bps3))
+                return set_error(ctx, MSA_ERR_CUDA, "occupancy query failed (no sm_100a image?)");
+            ctx->plain_blocks_per_sm = std::min(bps, bps3);
+        }
+        resident_blocks = (uint64_t) ctx->num_sms * (uint64_t) ctx->plain_blocks_per_sm;
+    }
     uint64_t warps_needed = resident_blocks * kWPB;
 
     // Persistent task tables: rows pairs (sorted 2k, 2k+1) x column groups of W.
@@ -1761,11 +1806,11 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
         };
         int rc;
         const uint64_t all_groups = tables(1);
-        if(ctx->nw_variant & MSA_NW_VARIANT_NO_PACKED) rc = batched_grid<32, 8, false>(ctx, all_groups, &pl->batch_grid);
-        else if(tiles.R == 16 && tiles.W == 4) rc = batched_grid<16, 4>(ctx, all_groups, &pl->batch_grid);
-        else if(tiles.R == 16 && tiles.W == 8) rc = batched_grid<16, 8>(ctx, all_groups, &pl->batch_grid);
-        else if(tiles.R == 32 && tiles.W == 4) rc = batched_grid<32, 4>(ctx, all_groups, &pl->batch_grid);
-        else rc = batched_grid<32, 8>(ctx, all_groups, &pl->batch_grid);
+        if(ctx->nw_variant & MSA_NW_VARIANT_NO_PACKED) rc = batched_grid<32, 8, false>(ctx, 0, all_groups, &pl->batch_grid);
+        else if(tiles.R == 16 && tiles.W == 4) rc = batched_grid<16, 4>(ctx, 1, all_groups, &pl->batch_grid);
+        else if(tiles.R == 16 && tiles.W == 8) rc = batched_grid<16, 8>(ctx, 2, all_groups, &pl->batch_grid);
+        else if(tiles.R == 32 && tiles.W == 4) rc = batched_grid<32, 4>(ctx, 3, all_groups, &pl->batch_grid);
+        else rc = batched_grid<32, 8>(ctx, 4, all_groups, &pl->batch_grid);
         if(rc) return rc;
         const uint32_t want = ctx->nw_chunk ? ctx->nw_chunk : pick_chunk(st, nclean);
         for(gchunk = want; gchunk > 1 && tables(gchunk) < 16 * pl->batch_grid; gchunk /= 2) {}
@@ -1775,32 +1820,30 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
         warps_needed = std::max<uint64_t>(warps_needed, pl->batch_grid * tiles.W);
     }
 
-    // One device allocation owned by the plan.
+    // One device block owned by the plan; the tables that come from the host
+    // lie at its start and are copied at once.
     size_t off = 0;
     auto take = [&off](size_t b) { size_t o = off; off = round_up(off + b, 256); return o; };
-    const size_t o_prof = take(st->prof_bytes + 64), o_ext = take(kAlpha * kAlpha),
-                 o_bound = take(warps_needed * stride * sizeof(uint32_t)), o_rt = take((K + 1) * sizeof(uint64_t)),
-                 o_rn = take(K + 16), o_co = take((K + 1) * sizeof(uint64_t)), o_cb = take(chain_words * sizeof(uint32_t)),
-                 o_gp = take(gpairs.size() * sizeof(uint32_t) + 16), o_ord = take(nclean * sizeof(uint32_t) + 16),
+    const size_t o_ext = take(kAlpha * kAlpha), o_rt = take((K + 1) * sizeof(uint64_t)), o_rn = take(K + 16),
+                 o_co = take((K + 1) * sizeof(uint64_t)), o_gp = take(gpairs.size() * sizeof(uint32_t) + 16),
+                 o_ord = take(nclean * sizeof(uint32_t) + 16), staged = off;
+    const size_t o_prof = take(st->prof_bytes + 64), o_bound = take(warps_needed * stride * sizeof(uint32_t)),
+                 o_cb = take(chain_words * sizeof(uint32_t)),
                  // the work counter, the error word and the chained strips' progress, cleared by every launch
                  o_cnt = take(64 + chain_tasks * 8 * sizeof(uint32_t));
-    MSA_CUDA_TRY(ctx, pl->mem.ensure(off));
-    char *base = (char *) pl->mem.ptr;
+    MSA_CUDA_TRY(ctx, ctx->blocks.take(off, &pl->mem, &pl->mem_bytes));
+    pl->home = ctx;
+    char *base = (char *) pl->mem;
     cudaStream_t s = ctx->stream;
-    MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_ext, tbl.score, kAlpha * kAlpha, cudaMemcpyHostToDevice, s));
-    if(K) {
-        MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_rt, row_task.data(), (K + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
-        MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_rn, row_narrow.data(), K, cudaMemcpyHostToDevice, s));
-        if(chain_tasks)
-            MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_co, chain_off.data(), (K + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
-    }
-    if(nclean)
-        MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_ord, st->clean_sorted.data(), nclean * sizeof(uint32_t),
-                                          cudaMemcpyHostToDevice, s));
-    if(!gpairs.empty())
-        MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_gp, gpairs.data(), gpairs.size() * sizeof(uint32_t),
-                                          cudaMemcpyHostToDevice, s));
-    MSA_CUDA_TRY(ctx, cudaStreamSynchronize(s));   // host vectors go out of scope
+    pl->staged.assign(staged, 0);
+    auto put = [&](size_t o, const void *src, size_t b) { if(b) std::memcpy(pl->staged.data() + o, src, b); };
+    put(o_ext, tbl.score, kAlpha * kAlpha);
+    put(o_rt, row_task.data(), row_task.size() * sizeof(uint64_t));
+    put(o_rn, row_narrow.data(), row_narrow.size());
+    put(o_co, chain_off.data(), chain_off.size() * sizeof(uint64_t));
+    put(o_gp, gpairs.data(), gpairs.size() * sizeof(uint32_t));
+    put(o_ord, st->clean_sorted.data(), nclean * sizeof(uint32_t));
+    MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base, pl->staged.data(), staged, cudaMemcpyHostToDevice, s));
 
     pl->d_ext = (const int8_t *) (base + o_ext);
     NwParams &p = pl->p;
@@ -1941,7 +1984,15 @@ int nw_run(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode, int32_t *d
         }
     }
     if(!pl) {
-        while(plans.size() >= kMaxPlans) { delete plans.front(); plans.erase(plans.begin()); }
+        auto held = [&plans] {
+            size_t b = 0;
+            for(const NwPlan *c : plans) b += c->mem_bytes;
+            return b;
+        };
+        while(!plans.empty() && (plans.size() >= kMaxPlans || held() > kMaxPlanBytes)) {
+            ctx->graphs->drop(plans.front());
+            plans.erase(plans.begin());
+        }
         pl = new NwPlan;
         const int rc = build_plan(ctx, st, tbl, mode, d_out, tiles, part, nparts, pl);
         if(rc) { delete pl; return rc; }
@@ -1960,7 +2011,7 @@ int nw_run(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode, int32_t *d
             e = cudaStreamEndCapture(s, &g);
             if(!e) e = e2;
         }
-        if(!e) e = cudaGraphInstantiate(&pl->exec, g, 0);
+        if(!e) e = ctx->graphs->instantiate(g, &pl->exec);
         if(g) cudaGraphDestroy(g);
         if(e) {
             cudaGetLastError();

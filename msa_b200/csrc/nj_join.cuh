@@ -67,6 +67,7 @@ namespace njdev {
 
 constexpr int kJoinThreads = 512;
 constexpr int kJoinWarps = kJoinThreads / 32;
+static_assert(kJoinWarps == 16, "half a warp reads one candidate per warp");
 constexpr int kFoldWarps = 2;                   // fold a row sum while the others scan
 constexpr int kScanWarps = kJoinWarps - kFoldWarps;
 constexpr int kFoldParts = kFoldWarps * 8;      // four lanes each
@@ -120,7 +121,7 @@ struct Joined {
 };
 
 // raise_candidate (sequential.cpp:142-152).
-__device__ __forceinline__ void record_join(const Stage &st, uint32_t at, const Joined &j)
+__device__ __noinline__ void record_join(uint32_t *rec_x, uint32_t *rec_y, float *rec_dx, float *rec_dy, const Joined &j)
 {
     const float pairsum = __fsub_rn(j.sx, j.sy);
     const float den = (float) (2u * (j.c - 2));
@@ -132,10 +133,10 @@ __device__ __forceinline__ void record_join(const Stage &st, uint32_t at, const 
     // and dy, where the GPU would give its canonical 0x7FFFFFFF.
     if(dx != dx) dx = __uint_as_float(0xFFC00000u);
     if(dy != dy) dy = __uint_as_float(0xFFC00000u);
-    st.rec_x[at] = j.x;
-    st.rec_y[at] = j.y;
-    st.rec_dx[at] = dx;
-    st.rec_dy[at] = dy;
+    *rec_x = j.x;
+    *rec_y = j.y;
+    *rec_dx = dx;
+    *rec_dy = dy;
 }
 
 // The serial fold of a new row sum over values V[i], i ascending, as a float
@@ -144,7 +145,7 @@ __device__ __forceinline__ void record_join(const Stage &st, uint32_t at, const 
 // of 4 with -0 (x + -0 = x).
 __device__ __forceinline__ float fold_serial(const float *V, uint32_t lo, uint32_t hi, float s)
 {
-#pragma unroll 8
+#pragma unroll 4
     for(uint32_t i = lo; i < hi; i += 4) {
         const float4 v = *reinterpret_cast<const float4 *>(V + i);
         s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v.x), v.y), v.z), v.w);
@@ -152,10 +153,14 @@ __device__ __forceinline__ float fold_serial(const float *V, uint32_t lo, uint32
     return s;
 }
 
+// The same out of line, where it is rare.
+__device__ __noinline__ float fold_again(const float *V, uint32_t lo, uint32_t hi, float s) { return fold_serial(V, lo, hi, s); }
+
 // The literal double chain over 0.5 W[i] (some value is not a float).
-__device__ __forceinline__ float fold_wide(const float *W, uint32_t n)
+__device__ __noinline__ float fold_wide(const float *W, uint32_t n)
 {
     float s = 0.0f;
+#pragma unroll 1
     for(uint32_t i = 0; i < n; ++i) s = __double2float_rn(__dadd_rn((double) s, 0.5 * (double) W[i]));
     return s;
 }
@@ -178,6 +183,7 @@ __device__ __forceinline__ float fold_parts(const float *V, uint32_t n, float4 *
     const uint32_t len = ((n + kFoldParts - 1) / kFoldParts + 3) & ~3u, n4 = (n + 3) & ~3u;
     const uint32_t lo = min(g * len, n4), hi = min(lo + len, n4);
     float e = 0.0f;
+#pragma unroll 4
     for(uint32_t i = lo + 4 * r; i < hi; i += 16) {
         const float4 v = *reinterpret_cast<const float4 *>(V + i);
         e += (v.x + v.y) + (v.z + v.w);
@@ -238,11 +244,12 @@ __device__ __forceinline__ float fold_parts(const float *V, uint32_t n, float4 *
         }
         if(!ok) {
             t = 0.0f;
+#pragma unroll 1
             for(uint32_t k = 0; k < kFoldParts; ++k) {
                 const float4 p = fp[4 * k + (k ? (__float_as_uint(t) & 3u) : 0u)];
                 const float d = __fsub_rn(t, p.x);
                 const uint32_t a = min(k * len, n4);
-                t = d == 0.0f || fabsf(d) <= p.z ? __fadd_rn(p.y, d) : fold_serial(V, a, min(a + len, n4), t);
+                t = d == 0.0f || fabsf(d) <= p.z ? __fadd_rn(p.y, d) : fold_again(V, a, min(a + len, n4), t);
             }
         }
     }
@@ -312,6 +319,7 @@ __device__ __forceinline__ RowScan scan_row(const float *__restrict__ row, const
     RowScan r{-INFINITY, -INFINITY, 0.0f, 3.0e38f, kDead};
     const float si = S[i];
     const uint32_t pi = pos[i], nch = P >> 2, stride = 32 * wpr;
+#pragma unroll 1
     for(uint32_t g0 = sub * 32 + lane; g0 < nch; g0 += kRowBatch * stride) {
         float4 d[kRowBatch];
 #pragma unroll
@@ -343,7 +351,9 @@ __device__ __forceinline__ RowScan scan_row(const float *__restrict__ row, const
     }
     if(r.m1 == r.m2 && r.j1 != kDead) {
         uint32_t first = pos[r.j1];
+#pragma unroll 1
         for(uint32_t g = sub * 32 + lane; g < nch; g += stride)
+#pragma unroll 1
             for(uint32_t j = 4 * g; j < 4 * g + 4; ++j) {
                 const uint32_t pj = pos[j];
                 if(S[j] == INFINITY || pj == pi) continue;
@@ -359,7 +369,7 @@ __device__ __forceinline__ RowScan scan_row(const float *__restrict__ row, const
 }
 
 // The lanes' scans of one row (logical index pi) as one; every lane gets it.
-__device__ __forceinline__ RowScan merge_scans(const RowScan &r, const uint16_t *pos, uint32_t pi, int lane)
+__device__ __noinline__ RowScan merge_scans(const RowScan &r, const uint16_t *pos, uint32_t pi, int lane)
 {
     RowScan o;
     o.m1 = warp_fmax(r.m1);
@@ -415,6 +425,10 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
     if(*st.err != 0) return;   // an earlier launch failed (the same for every CTA)
     float *D = st.D;
 
+    auto record = [&](uint32_t k) {
+        const uint32_t at = st.step0 + k;
+        record_join(st.rec_x + at, st.rec_y + at, st.rec_dx + at, st.rec_dy + at, joined);
+    };
     auto scan_sync = [] { asm volatile("barrier.sync 1, %0;" ::"n"(kScanWarps * 32) : "memory"); };
     // Size of values that Q is made of, as float bits (a NaN is the largest):
     // N |D| and 2 |S|; bit 0 marks a new distance that is not a float.
@@ -464,12 +478,6 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
             t_last = now;
         }
     };
-    // The new node's row sum over the c values of its join, by the folding warps.
-    auto fold = [&](uint32_t n) {
-        if(exact) return fold_parts(NDl, n, fparts, fsum, tid);
-        return warp == 0 ? fold_wide(Wl, n) : 0.0f;
-    };
-
     while(c > st.c_end) {
         const float cm2 = (float) (c - 2), size = __uint_as_float(sv);
         const bool prune = size < 1e30f;
@@ -487,7 +495,8 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
         if(warp < kFoldWarps) {
             if(z != kDead) {
                 const uint32_t f0 = (uint32_t) clock64();
-                const float ns = fold(c + 1);
+                // Its row sum over the c + 1 values of its join.
+                const float ns = exact ? fold_parts(NDl, c + 1, fparts, fsum, tid) : fold_wide(Wl, c + 1);
                 if(tid == 0) {
                     sz_sh = ns;
                     cyc_fold += (uint32_t) clock64() - f0;
@@ -495,7 +504,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
             }
         } else {
             const uint32_t w = (uint32_t) warp - kFoldWarps, sid = (uint32_t) tid - 32 * kFoldWarps;
-            if(rank == 0 && step > 0 && tid == kJoinThreads - 1) record_join(st, st.step0 + step - 1, joined);
+            if(rank == 0 && step > 0 && tid == kJoinThreads - 1) record(step - 1);
             // A Q that some live pair attains, from what is left of the last
             // search: this CTA's candidates by warp and every CTA's.
             float L = -INFINITY;
@@ -508,6 +517,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
                 }
                 L = warp_fmax(L);
             }
+#pragma unroll 1
             for(uint32_t l = sid; l < own; l += kScanWarps * 32) {
                 const uint32_t i = l * K + rank;
                 if(i > N || pos[i] == kDead || i == z) continue;
@@ -526,26 +536,27 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
                 tau[l] = (uint16_t) step;
                 Zb[l] = stored(__fadd_ru(r.m2, slack), S[l * K + rank]);
             };
-            // Warps per row: as many as there are, down to one load a lane each.
-            const uint32_t wpr = min(m ? kScanWarps / m : 1u, (P + 127) / 128);
-            if(wpr <= 1) {
-                for(uint32_t k = w; k < m; k += kScanWarps) {
-                    const uint32_t l = list[k], i = l * K + rank;
-                    renew(l, merge_scans(scan_row(D + (size_t) i * P, S, pos, i, P, cm2, 0, 1, lane), pos, pos[i], lane));
-                }
-            } else {
-                const uint32_t k = w / wpr;
-                if(k < m) {
-                    const uint32_t i = list[k] * K + rank;
-                    const RowScan o = merge_scans(
-                        scan_row(D + (size_t) i * P, S, pos, i, P, cm2, w - k * wpr, wpr, lane), pos, pos[i], lane);
+            // Warps per row, a power of two: as many as there are for m rows,
+            // down to one load a lane each.
+            const uint32_t lg = min(m <= 1 ? 3u : m <= 3 ? 2u : m <= 7 ? 1u : 0u, P > 512 ? 3u : P > 256 ? 2u : 1u);
+            const uint32_t wpr = 1u << lg, rows = kScanWarps >> lg;   // rows scanned at once
+#pragma unroll 1
+            for(uint32_t k = w >> lg; k < m; k += rows) {   // once where warps share a row: m <= rows
+                const uint32_t l = list[k], i = l * K + rank;
+                const RowScan o = merge_scans(
+                    scan_row(D + (size_t) i * P, S, pos, i, P, cm2, w & (wpr - 1), wpr, lane), pos, pos[i], lane);
+                if(wpr > 1) {
                     if(lane == 0) wscan[w] = o;
+                } else {
+                    renew(l, o);
                 }
+            }
+            if(wpr > 1) {
                 scan_sync();
                 if(w < m) {
                     const uint32_t l = list[w], i = l * K + rank;
                     RowScan r{-INFINITY, -INFINITY, 0.0f, 3.0e38f, kDead};
-                    if((uint32_t) lane < wpr) r = wscan[w * wpr + lane];
+                    if((uint32_t) lane < wpr) r = wscan[(w << lg) + lane];
                     renew(l, merge_scans(r, pos, pos[i], lane));
                 }
             }
@@ -562,6 +573,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
                 nlist = 0;
             }
             Cand best = no_cand();
+#pragma unroll 1
             for(uint32_t l = tid; l < own; l += kJoinThreads) {
                 const uint32_t i = l * K + rank, pi = i <= N ? pos[i] : kDead;
                 if(pi == kDead || i == z) continue;
@@ -627,10 +639,12 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
         const float *rx = D + (size_t) X * P, *ry = D + (size_t) Y * P;
         float fall = -INFINITY;
         bool ex = true;
+        uint32_t moved = kDead;
         if((uint32_t) tid < ((4u - (c & 3u)) & 3u)) NDl[c + tid] = -0.0f;
         // join_pair (sequential.cpp:247-267) for every live slot; X and Y read
         // the diagonal and D[x][y], as the reference does.
         constexpr int U = 4;
+#pragma unroll 1
         for(uint32_t s0 = tid; s0 <= N; s0 += U * kJoinThreads) {
             float a[U], b[U];
             uint32_t p[U];
@@ -654,43 +668,46 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
                 Wl[p[u] - t] = w;
                 NDl[p[u] - t] = nd;
                 if((s & (K - 1)) == rank) ND[s >> kbits] = nd;
-                const bool mine = ((s >> 5) & (K - 1)) == rank;
-                if(s == Y) {
-                    if(rank == 0) joined = Joined{S[X], S[Y], dxy, x, y, c};
-                    S[X] = INFINITY;
-                    S[Y] = INFINITY;
-                    pos[Y] = (uint16_t) kDead;
-                } else if(s == X) {
-                    const uint32_t pz = px == ps ? py : px;
-                    pos[X] = (uint16_t) kDead;
-                    pos[znew] = (uint16_t) pz;
-                    l2s[pz] = (uint16_t) znew;
-                    S[znew] = INFINITY;   // until its row sum is folded and its column is written
-                    if(mine) D[(size_t) znew * P + znew] = nd;   // its diagonal
-                    if((znew & (K - 1)) == rank) {
-                        // Nothing is covered by the new node's own row yet.
-                        const uint32_t l = znew >> kbits;
-                        Zb[l] = -INFINITY;
-                        Dm[l] = 3.0e38f;
-                        jb[l] = (uint16_t) kDead;
-                        tau[l] = (uint16_t) (step + 1);
-                    }
-                } else {
-                    if(p[u] == ps) {
-                        pos[s] = (uint16_t) py;
-                        l2s[py] = (uint16_t) s;
-                    }
-                    const float s_old = S[s];
-                    const double uu = __dmul_rn((double) w, 0.5);
-                    const float sn = __double2float_rn(__dadd_rn((double) s_old, __dsub_rn(uu, (double) prev)));
-                    S[s] = sn;
-                    fall = fmaxf(fall, __fsub_ru(s_old, sn));
-                    sv = max(sv, size_of(nd, sn));
-                    if(mine) {
-                        D[(size_t) znew * P + s] = nd;
-                        D[(size_t) s * P + znew] = nd;
-                    }
+                if(p[u] == ps) moved = s;
+                if(s == X || s == Y) continue;   // their numbers and sums below
+                const float s_old = S[s];
+                const double uu = __dmul_rn((double) w, 0.5);
+                const float sn = __double2float_rn(__dadd_rn((double) s_old, __dsub_rn(uu, (double) prev)));
+                S[s] = sn;
+                fall = fmaxf(fall, __fsub_ru(s_old, sn));
+                sv = max(sv, size_of(nd, sn));
+                if(((s >> 5) & (K - 1)) == rank) {
+                    D[(size_t) znew * P + s] = nd;
+                    D[(size_t) s * P + znew] = nd;
                 }
+            }
+        }
+        // The node that changes its number: its thread alone reads pos here.
+        if(moved != kDead && moved != X && moved != Y) {
+            pos[moved] = (uint16_t) py;
+            l2s[py] = (uint16_t) moved;
+        }
+        if((uint32_t) tid == (Y & (kJoinThreads - 1))) {
+            if(rank == 0) joined = Joined{S[X], S[Y], dxy, x, y, c};
+            S[X] = INFINITY;
+            S[Y] = INFINITY;
+            pos[Y] = (uint16_t) kDead;
+        }
+        if((uint32_t) tid == (X & (kJoinThreads - 1))) {
+            const uint32_t pz = px == ps ? py : px;
+            pos[X] = (uint16_t) kDead;
+            pos[znew] = (uint16_t) pz;
+            l2s[pz] = (uint16_t) znew;
+            S[znew] = INFINITY;   // until its row sum is folded and its column is written
+            // Its diagonal, as the join gives it for x.
+            if(rank == 0) D[(size_t) znew * P + znew] = NDl[px - t];
+            if((znew & (K - 1)) == rank) {
+                // Nothing is covered by the new node's own row yet.
+                const uint32_t l = znew >> kbits;
+                Zb[l] = -INFINITY;
+                Dm[l] = 3.0e38f;
+                jb[l] = (uint16_t) kDead;
+                tau[l] = (uint16_t) (step + 1);
             }
         }
         fall = warp_fmax(fall);
@@ -718,11 +735,11 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
     }
     if(rank == 0) {
         if(!failed && !bad) {
-            if(tid == kJoinThreads - 1) record_join(st, st.step0 + step - 1, joined);
+            if(tid == kJoinThreads - 1) record(step - 1);
             // What the next launch starts from.
-            if(warp < kFoldWarps) {
-                const float ns = fold(c + 1);
-                if(tid == 0) S[z] = ns;
+            if(warp == 0) {
+                const float ns = exact ? fold_again(NDl, 0, (c + 4) & ~3u, 0.0f) : fold_wide(Wl, c + 1);
+                if(lane == 0) S[z] = ns;
             }
             __syncthreads();
             for(uint32_t k = tid; k < c; k += kJoinThreads) {
@@ -786,8 +803,10 @@ __global__ void __launch_bounds__(kThreads, 1) nj_small_kernel(Stage st)
 
     if(st.tri) {
         // A warp per row of the triangle.
+#pragma unroll 1
         for(uint32_t i = 1 + warp; i < N; i += kWarps) {
             const uint32_t at = i * (i - 1) / 2;
+#pragma unroll 2
             for(uint32_t j = lane; j < i; j += 32) {
                 const float v = st.tri_int ? (float) static_cast<const int32_t *>(st.tri)[at + j]
                                            : static_cast<const float *>(st.tri)[at + j];
@@ -817,6 +836,10 @@ __global__ void __launch_bounds__(kThreads, 1) nj_small_kernel(Stage st)
     for(uint32_t k = N + tid; k < P + 32 * kSmallCols; k += kThreads) S[k] = INFINITY;
     __syncthreads();
 
+    auto record = [&](uint32_t k) {
+        const uint32_t at = st.step0 + k;
+        record_join(st.rec_x + at, st.rec_y + at, st.rec_dx + at, st.rec_dy + at, joined);
+    };
     uint32_t c = N, t = 0, step = 0, z = kDead;
     bool exact = true;
     unsigned long long scan_cyc = 0, fold_cyc = 0, rest_cyc = 0, t_last = clock64();
@@ -830,12 +853,13 @@ __global__ void __launch_bounds__(kThreads, 1) nj_small_kernel(Stage st)
                 fold_cyc += clock64() - t_last;
             }
         } else {
-            if(tid == kThreads - 1 && step > 0) record_join(st, st.step0 + step - 1, joined);
+            if(tid == kThreads - 1 && step > 0) record(step - 1);
             float sb[kSmallCols];
 #pragma unroll
             for(int k = 0; k < kSmallCols; ++k) sb[k] = S[t + 32 * k + lane];
             float bq = -INFINITY;
             uint32_t bij = 0;
+#pragma unroll 1
             for(uint32_t a = warp; a < c; a += kWarps - 1) {
                 const float sa = S[t + a];
                 const float *row = D + (t + a) * P + t + lane;
@@ -945,7 +969,7 @@ __global__ void __launch_bounds__(kThreads, 1) nj_small_kernel(Stage st)
         }
         if(warp == 0) t_last = clock64();
     }
-    if(c == 1 && tid == kThreads - 1) record_join(st, st.step0 + step - 1, joined);
+    if(c == 1 && tid == kThreads - 1) record(step - 1);
     if(tid == 32) {
         atomicAdd(st.cycles + 0, scan_cyc);
         atomicAdd(st.cycles + 2, rest_cyc);

@@ -306,6 +306,11 @@ def nw_ceilings(wl, workload: str, nsm: int, sm_mhz: float, lds: float) -> tuple
         except Exception:
             traffic = inst = None
     f = packed_row_fraction(wl)
+    if wl.table == "default":
+        # Bit planes (nw_bits.cu): eight three-input logic operations on the ALU
+        # pipe and one shared-memory word per 32 cells.
+        c = {"alu": nsm * (64.0 * 32 / 8) * sm_mhz * 1e6 / 1e9, "smem": nsm * (lds / 4.0 * 32) * sm_mhz * 1e6 / 1e9}
+        return c, "alu", 0.0, None, None
     c = {"smem": nsm * (lds / (2.0 - f)) * sm_mhz * 1e6 / 1e9,
          "alu": nsm * (64.0 / ((1.0 + f) / 2.0)) * sm_mhz * 1e6 / 1e9}
     if inst:
@@ -963,38 +968,12 @@ def main():
         props = torch.cuda.get_device_properties(local)
         sm_mhz = clocks.get("sm_mhz") or 1965.0
         nsm = props.multi_processor_count
-        # DRAM traffic and counted instructions per cell of this kernel on this
-        # workload, from the committed ncu summaries.
-        traffic = inst_per_cell = None
-        tp = ROOT / "profiles" / "nw_traffic.json"
-        if tp.exists():
-            try:
-                tj = json.loads(tp.read_text())
-                traffic = tj.get(args.workload)
-                inst_per_cell = tj.get(args.workload + "_inst_per_cell")
-            except Exception:
-                traffic = inst_per_cell = None
-        # Ceilings of the batched kernel from rates measured here per SM clock
-        # (msa_probe_op). A cell reads its score from shared memory: 2 bytes in
-        # a 16-bit profile row, 1 byte in a packed row (a share f of the cells,
-        # from the kernel's plan), so 2 - f bytes per cell. The ALU pipe
-        # (64 lanes/clk/SM) carries one vimax3 per two cells and one PRMT per
-        # two cells of a packed row: (1 + f) / 2 lane-ops per cell. The lowest
-        # ceiling (these two, and issue below) is the roofline.
+        # Ceilings from rates measured here per SM clock (msa_probe_op); the
+        # lowest one is the roofline.
         lds = probe_rate(ctx, 15)
         cell_ops = probe_rate(ctx, 14)
-        f_packed = packed_row_fraction(wl)
-        smem_peak = nsm * (lds / (2.0 - f_packed)) * sm_mhz * 1e6 / 1e9
-        alu_peak = nsm * (64.0 / ((1.0 + f_packed) / 2.0)) * sm_mhz * 1e6 / 1e9
+        ceilings, bound, f_packed, inst_per_cell, traffic = nw_ceilings(wl, args.workload, nsm, sm_mhz, lds)
         cell_peak = nsm * (2.0 * cell_ops) * sm_mhz * 1e6 / 1e9
-        # Issue: 4 warp-instructions (128 lane-instructions) per SM per clock
-        # over the lane-instructions per cell that ncu counted for this kernel
-        # on this workload (profiles/nw_traffic.json), when there is a count.
-        issue_peak = nsm * (128.0 / inst_per_cell) * sm_mhz * 1e6 / 1e9 if inst_per_cell else None
-        ceilings = {"smem": smem_peak, "alu": alu_peak}
-        if issue_peak:
-            ceilings["issue"] = issue_peak
-        bound = min(ceilings, key=ceilings.get)
         roof = ceilings[bound]
         # The four-op int32 issue figure (two max operations per cell on the ALU
         # pipe, 64 lanes/clk/SM): 32 cells/clk/SM.
@@ -1019,15 +998,17 @@ def main():
                          "peak": roof, "unit": "GCUPS", "frac": kernel_gcups / roof, "traffic": traffic,
                          "frac_int32_issue": kernel_gcups / peak,
                          "packed_row_fraction": f_packed, "inst_per_cell_counted": inst_per_cell,
-                         "ceilings_gcups": {"smem_profile_reads": smem_peak, "alu_pipe": alu_peak,
-                                            "issue_counted_instructions": issue_peak,
+                         "ceilings_gcups": {"smem_reads": ceilings["smem"], "alu_pipe": ceilings["alu"],
+                                            "issue_counted_instructions": ceilings.get("issue"),
                                             "cell_ops_16x2_probe": cell_peak, "int32_issue_4ops_per_cell": peak},
                          "measured_per_sm_clk": {"lds_bytes": lds, "cell_16x2_lane_ops": cell_ops},
-                         "peak_basis": f"min of {nsm} SM x {lds:.1f} shared-memory bytes/clk (measured, "
-                                       f"ld.shared.v4) / (2 - {f_packed:.3f}) bytes of profile per cell, "
-                                       f"{nsm} SM x 64 ALU lanes/clk / ((1 + {f_packed:.3f}) / 2) lane-ops per cell"
-                                       + (f" and {nsm} SM x 128 issued lane-instructions/clk / {inst_per_cell} "
-                                          f"counted per cell" if inst_per_cell else "")
+                         "peak_basis": (f"{nsm} SM x 64 ALU lanes/clk x 32 cells / 8 logic operations"
+                                        if wl.table == "default" else
+                                        f"min of {nsm} SM x {lds:.1f} shared-memory bytes/clk (measured, "
+                                        f"ld.shared.v4) / (2 - {f_packed:.3f}) bytes of profile per cell, "
+                                        f"{nsm} SM x 64 ALU lanes/clk / ((1 + {f_packed:.3f}) / 2) lane-ops per cell"
+                                        + (f" and {nsm} SM x 128 issued lane-instructions/clk / {inst_per_cell} "
+                                           f"counted per cell" if inst_per_cell else ""))
                                        + f", x {sm_mhz:.0f} MHz (median sampled); frac_int32_issue is against "
                                          f"{nsm} SM x 64 ALU lanes/clk / 2 max-ops per cell"},
             "clocks": clocks,

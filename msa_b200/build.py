@@ -17,8 +17,8 @@ LIB = PKG / "libmsa_b200.so"
 BUILD_DIR = PKG / "_build"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-SOURCES = ["tables.cpp", "abi.cpp", "partition.cpp", "nw_kernels.cu", "nj_kernel.cu", "probe.cu", "noalloc.cu",
-           "serve.cpp", "facade.cu", "fasta.cpp"]
+SOURCES = ["tables.cpp", "abi.cpp", "partition.cpp", "nw_kernels.cu", "nw_bits.cu", "nj_kernel.cu", "probe.cu",
+           "noalloc.cu", "serve.cpp", "facade.cu", "fasta.cpp"]
 # The command line (museqa), linked against the library.
 CLI = PKG / "museqa"
 CLI_SOURCE = "cli.cpp"

@@ -122,6 +122,7 @@ struct msa_ctx {
     msa::BlockCache blocks;
     int plain_blocks_per_sm = 0;      // of the per-warp kernels, once asked for
     int batch_blocks_per_sm[5] = {};  // of the batched kernel's instances
+    int bits_blocks_per_sm = 0;       // of the bit-plane kernel
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     std::string err;

@@ -26,7 +26,7 @@
 #include <cstring>
 #include <type_traits>
 
-#include "msa_internal.hpp"
+#include "nw_bits.hpp"
 
 namespace msa {
 namespace dev {
@@ -1529,6 +1529,8 @@ struct NwPlan {
     const int8_t *d_ext = nullptr;
     NwParams p{};
     BatchParams bp{};
+    BitParams bits{};           // of the pairs on bit planes, if any (ntasks > 0)
+    uint64_t bits_grid = 0;
     uint32_t n = 0;
     uint64_t ngeneric = 0, gen_blocks = 0;
     std::vector<PlainLaunch> plain;
@@ -1540,6 +1542,7 @@ struct NwPlan {
     uint32_t chunk = 0;         // and its groups-per-task override
     size_t clear_bytes = 64;    // of the work counter and what follows it
     bool chained = false;
+    bool profiles = true;       // whether any kernel of the plan reads score profiles
     cudaGraphExec_t exec = nullptr;
     cudaStream_t captured_on = nullptr;
     ~NwPlan()
@@ -1650,6 +1653,20 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     const uint32_t nclean = (uint32_t) st->clean_sorted.size();
     const uint64_t nclean_pairs = (uint64_t) nclean * (nclean > 0 ? nclean - 1 : 0) / 2;
 
+    // What runs on bit planes (nw_bits.cu): where the table allows it, pairs
+    // beyond the first 32 g0 sequences; `nrows` sequences are left to the
+    // batched kernel. Parts of a job and overridden tiles stay on that kernel.
+    BitPlan bits;
+    const BitTable planes = bit_table(tbl);
+    uint32_t nrows = nclean;
+    if(mode == MSA_NW_PERSISTENT && planes.u && nparts == 1 && nclean > 32 && !st->any_gap && !ctx->nw_variant &&
+       !ctx->tile_r && !ctx->nw_chunk) {
+        std::vector<uint32_t> eff(nclean);
+        for(uint32_t a = 0; a < nclean; ++a) eff[a] = st->eff[st->clean_sorted[a]];
+        bits = plan_bits(eff, (uint32_t) ctx->num_sms);
+        if(bits.ntasks) nrows = 32 * bits.g0;
+    }
+
     // Pairs with at least one dirty sequence, in the reference's orientation,
     // and this part's runs of rows pairs and generic pairs.
     std::vector<uint32_t> gpairs_all;
@@ -1704,18 +1721,19 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     uint32_t K = 0;
     uint64_t task_base = 0;
     uint32_t gchunk = 1;
-    if(mode == MSA_NW_PERSISTENT && nclean_pairs > 0) {
-        K = (nclean + 1) / 2;
+    if(mode == MSA_NW_PERSISTENT && nclean_pairs > 0 && nrows > 1) {
+        K = (nrows + 1) / 2;
+        const uint32_t k_hi = std::min(split.k[part + 1], K);
         const int SH = 32 * tiles.R;
         const bool gap = st->any_gap;
-        auto eff_at = [&](uint32_t a) { return (uint64_t) st->eff[st->clean_sorted[std::min(a, nclean - 1)]]; };
+        auto eff_at = [&](uint32_t a) { return (uint64_t) st->eff[st->clean_sorted[std::min(a, nrows - 1)]]; };
         // Rows of rows pair k, and its longest column sequence.
         auto rows_at = [&](uint32_t k) { return std::max(eff_at(2 * k), eff_at(2 * k + 1)); };
         auto cols_at = [&](uint32_t k) { return gap || !table_is_symmetric(tbl) ? (eff_at(2 * k + 1) + 2) / 3 * 3 : eff_at(2 * k + 1); };
         row_narrow.assign(K, 0);
         std::vector<uint64_t> groups_k(K, 0);
         for(uint32_t k = 0; k < K; ++k) {
-            const int64_t ncol = (int64_t) nclean - (2 * (int64_t) k + 1);
+            const int64_t ncol = (int64_t) nrows - (2 * (int64_t) k + 1);
             if(ncol <= 0) continue;
             const bool nar = narrow_ok((int64_t) round_up(rows_at(k), SH), (int64_t) cols_at(k), tbl, gap) && !(ctx->nw_variant & MSA_NW_VARIANT_INT32);
             row_narrow[k] = nar ? kRowNarrow : 0;
@@ -1739,7 +1757,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
             auto stack = [&](uint32_t pairs, uint32_t rows, uint8_t flag) {
                 if(groups_all < pairs * fill) return;
                 for(uint32_t k = k_lo; k + pairs <= k_hi;) {
-                    bool ok = 2 * ((uint64_t) k + pairs) <= nclean;
+                    bool ok = 2 * ((uint64_t) k + pairs) <= nrows;
                     for(uint32_t p = 0; p < pairs; ++p)
                         ok = ok && row_narrow[k + p] == kRowNarrow && groups_k[k + p] != 0 && rows_at(k + p) <= rows;
                     if(!ok) {
@@ -1820,15 +1838,25 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
         warps_needed = std::max<uint64_t>(warps_needed, pl->batch_grid * tiles.W);
     }
 
+    if(bits.ntasks) {
+        const int rc = bits_grid(ctx, bits, &pl->bits_grid);
+        if(rc) return rc;
+        pl->narrow_tasks += (uint32_t) bits.ntasks;
+    }
+
     // One device block owned by the plan; the tables that come from the host
     // lie at its start and are copied at once.
     size_t off = 0;
     auto take = [&off](size_t b) { size_t o = off; off = round_up(off + b, 256); return o; };
     const size_t o_ext = take(kAlpha * kAlpha), o_rt = take((K + 1) * sizeof(uint64_t)), o_rn = take(K + 16),
                  o_co = take((K + 1) * sizeof(uint64_t)), o_gp = take(gpairs.size() * sizeof(uint32_t) + 16),
-                 o_ord = take(nclean * sizeof(uint32_t) + 16), staged = off;
-    const size_t o_prof = take(st->prof_bytes + 64), o_bound = take(warps_needed * stride * sizeof(uint32_t)),
-                 o_cb = take(chain_words * sizeof(uint32_t)),
+                 o_ord = take(nclean * sizeof(uint32_t) + 16), o_bs = take(bits.sets.size() * sizeof(BitSet) + 16),
+                 o_go = take(bits.goff.size() * sizeof(uint64_t) + 16),
+                 o_gc = take(bits.gcols.size() * sizeof(uint32_t) + 16), staged = off;
+    pl->profiles = mode != MSA_NW_PERSISTENT || ntasks || pl->ngeneric;
+    const size_t o_prof = take((pl->profiles ? st->prof_bytes : 0) + 64), o_bound = take(warps_needed * stride * sizeof(uint32_t)),
+                 o_cb = take(chain_words * sizeof(uint32_t)), o_match = take(bits.match_words * sizeof(uint32_t)),
+                 o_bb = take(pl->bits_grid * kBitWarps * bits.bound_words * sizeof(uint2)),
                  // the work counter, the error word and the chained strips' progress, cleared by every launch
                  o_cnt = take(64 + chain_tasks * 8 * sizeof(uint32_t));
     MSA_CUDA_TRY(ctx, ctx->blocks.take(off, &pl->mem, &pl->mem_bytes));
@@ -1843,6 +1871,11 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     put(o_co, chain_off.data(), chain_off.size() * sizeof(uint64_t));
     put(o_gp, gpairs.data(), gpairs.size() * sizeof(uint32_t));
     put(o_ord, st->clean_sorted.data(), nclean * sizeof(uint32_t));
+    if(bits.ntasks) {
+        put(o_bs, bits.sets.data(), bits.sets.size() * sizeof(BitSet));
+        put(o_go, bits.goff.data(), bits.goff.size() * sizeof(uint64_t));
+        put(o_gc, bits.gcols.data(), bits.gcols.size() * sizeof(uint32_t));
+    }
     MSA_CUDA_TRY(ctx, cudaMemcpyAsync(base, pl->staged.data(), staged, cudaMemcpyHostToDevice, s));
 
     pl->d_ext = (const int8_t *) (base + o_ext);
@@ -1872,7 +1905,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     bp.job.poff = st->d_prof_off;
     bp.job.plp = st->d_prof_lp;
     bp.job.sorted = p.sorted;
-    bp.job.nclean = nclean;
+    bp.job.nclean = nrows;
     bp.job.row_narrow = (const uint8_t *) (base + o_rn);
     bp.job.out = d_out;
     bp.job.g = tbl.penalty;
@@ -1890,9 +1923,35 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     bp.chain_off = (const uint64_t *) (base + o_co);
     bp.step = (uint32_t) std::min<int64_t>(largest_step(tbl, st->any_gap), 0xffff);
     pl->clear_bytes = 64 + chain_tasks * 8 * sizeof(uint32_t);
-    pl->chained = chain_tasks != 0;
+    pl->chained = chain_tasks != 0 || bits.nchain != 0;
 
-    pl->launches = 1 + (pl->ngeneric ? 1 : 0);
+    if(bits.ntasks) {
+        BitParams &q = pl->bits;
+        q.units = st->d_units;
+        q.uoff = st->d_off;
+        q.eff = st->d_eff;
+        q.sorted = p.sorted;
+        q.nclean = nclean;
+        q.ngroups = (uint32_t) bits.gcols.size();
+        q.g0 = bits.g0;
+        q.sets = (const BitSet *) (base + o_bs);
+        q.nsets = (uint32_t) bits.sets.size();
+        q.ntasks = (uint32_t) bits.ntasks;
+        q.match = (uint32_t *) (base + o_match);
+        q.goff = (const uint64_t *) (base + o_go);
+        q.gcols = (const uint32_t *) (base + o_gc);
+        q.bound = (uint2 *) (base + o_bb);
+        q.bound_words = bits.bound_words;
+        q.out = d_out;
+        q.u = planes.u;
+        q.letters = planes.letters;
+        q.g = tbl.penalty;
+        q.nchain = (uint32_t) bits.nchain;
+        q.err = bp.err;
+        q.counter = (unsigned long long *) (base + o_cnt + 16);   // cleared with the batched kernel's
+    }
+
+    pl->launches = (pl->profiles ? 1 : 0) + (pl->ngeneric ? 1 : 0) + (bits.ntasks ? 2 : 0);
     if(mode == MSA_NW_PLAIN && nclean_pairs > 0) {
         // Buckets: runs of sorted rows with the same strip count.
         constexpr int SH = 32 * kPlainR;
@@ -1922,9 +1981,14 @@ static cudaError_t enqueue(msa_ctx *ctx, const NwPlan &pl, const SeqStore *st, c
     const unsigned flags = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
     cudaError_t e = cudaEventRecordWithFlags(ctx->ev[0], s, flags);
     if(e) return e;
-    build_profiles_kernel<<<pl.n, 256, 0, s>>>(st->d_units, st->d_off, st->d_eff, st->d_prof_off, st->d_prof_lp,
-                                               pl.d_ext, const_cast<int8_t *>(pl.p.prof));
-    if((e = cudaGetLastError())) return e;
+    if(pl.profiles) {
+        build_profiles_kernel<<<pl.n, 256, 0, s>>>(st->d_units, st->d_off, st->d_eff, st->d_prof_off, st->d_prof_lp,
+                                                   pl.d_ext, const_cast<int8_t *>(pl.p.prof));
+        if((e = cudaGetLastError())) return e;
+    }
+    if(pl.bits.ntasks) {
+        if((e = launch_match(pl.bits, s))) return e;
+    }
     if((e = cudaEventRecordWithFlags(ctx->ev[1], s, flags))) return e;
     const size_t smem = smem_bytes<kPlainR>();
     if(pl.ngeneric) {
@@ -1936,8 +2000,11 @@ static cudaError_t enqueue(msa_ctx *ctx, const NwPlan &pl, const SeqStore *st, c
             nw_plain_kernel<kPlainR, kWPB><<<(unsigned) L.blocks, kWPB * 32, smem, s>>>(pl.p, L.k_lo, L.k_hi);
             if((e = cudaGetLastError())) return e;
         }
-    } else if(pl.bp.ntasks) {
+        return cudaEventRecordWithFlags(ctx->ev[2], s, flags);
+    }
+    if(pl.bp.ntasks || pl.bits.ntasks)
         if((e = cudaMemsetAsync(pl.bp.counter, 0, pl.clear_bytes, s))) return e;
+    if(pl.bp.ntasks) {
         const Tiles t = pl.tiles;
         if(pl.variant & MSA_NW_VARIANT_NO_PACKED) launch_batched<32, 8, false>(pl, s);
         else if(t.R == 16 && t.W == 4) launch_batched<16, 4>(pl, s);
@@ -1945,6 +2012,9 @@ static cudaError_t enqueue(msa_ctx *ctx, const NwPlan &pl, const SeqStore *st, c
         else if(t.R == 32 && t.W == 4) launch_batched<32, 4>(pl, s);
         else launch_batched<32, 8>(pl, s);
         if((e = cudaGetLastError())) return e;
+    }
+    if(pl.bits.ntasks) {
+        if((e = launch_bits(pl.bits, pl.bits_grid, s))) return e;
     }
     return cudaEventRecordWithFlags(ctx->ev[2], s, flags);
 }

@@ -17,7 +17,7 @@
 // kernel is the ALU pipe (64 lanes per SM and clock, so 74 TCUPS at 1,965 MHz; ncu:
 // 84% busy on 3,000 reads, three in four of its instructions in cells).
 // 3,000 DNA reads of 100 to 250 bases 9.0 -> 2.96 ms, 1,200 uneven DNA sequences of
-// 200 to 16,000 bases 177 -> 71 ms.
+// 200 to 16,000 bases 177 -> 65 ms.
 //
 // A task is a set of 1, 2 or 4 rows sequences against one group of 32 sequences
 // that are neighbours in the length order; one warp runs it. Lanes own R
@@ -438,14 +438,17 @@ BitPlan plan_bits(const std::vector<uint32_t> &eff, uint32_t num_sms)
             cells[a / 32 + 1] = got;
         }
     }
-    constexpr double kShare = 2;   // a warp's pace beside two others on its scheduler
+    // A warp's pace beside three others on its scheduler. Taken as 2, 1,200 uneven
+    // sequences put the longest 32 against themselves here: 71 ms, most of it that task.
+    constexpr double kShare = 4;
+    auto rounds = [](const BitSet &s) { return (s.nst + kBitWarps - 1) / kBitWarps; };
     const double hz = 1.9e9, med = eff[n / 2], whole = med < 384 ? 11e12 : med < 1024 ? 13e12 : med < 2048 ? 15e12 : 16e12;
     double best = cells[ng] / whole;
     bp.g0 = ng;
     for(uint32_t q = 0; q < ng; ++q) {
         if(bp.gcols[q] > kBitMaxCols) continue;
         double serial = 0;   // the longest task: of the first set, or of a later group's own
-        if(!bp.sets.empty()) serial = kShare * rate(bp.sets[0]) * steps(bp.sets[0], q) / std::min<uint32_t>(bp.sets[0].nst, kBitWarps);
+        if(!bp.sets.empty()) serial = kShare * rate(bp.sets[0]) / bp.sets[0].nst * rounds(bp.sets[0]) * steps(bp.sets[0], q);
         const double both = q ? cells[q] / 10e12 + 20e-6 : 0;   // profiles, and another kernel's start and tail
         const double t = both + std::max(work[q] / (4.0 * num_sms), serial) / hz + 10e-6;
         if(t < best) best = t, bp.g0 = q;
@@ -459,10 +462,10 @@ BitPlan plan_bits(const std::vector<uint32_t> &eff, uint32_t num_sms)
         bp.ntasks += ng - q;
         bp.bound_words = std::max(bp.bound_words, 32 / s.lanes * (uint64_t) bit_bound(widest[q]));
     }
-    // The tasks that would take more than a quarter of the launch on one warp are
-    // chained. Sets are in falling order of length.
+    // The tasks that would take more than half of the launch on one warp are chained
+    // (a quarter and the whole of it measured within 2%). Sets are in falling order of length.
     for(const BitSet &s : bp.sets) {
-        if(s.nst < 2 || kShare * rate(s) * steps(s, std::max(bp.g0, s.a / 32)) < work[bp.g0] / (16.0 * num_sms)) break;
+        if(s.nst < 2 || kShare * rate(s) * steps(s, std::max(bp.g0, s.a / 32)) < work[bp.g0] / (8.0 * num_sms)) break;
         bp.nchain = s.first + (ng - std::max(bp.g0, s.a / 32));
     }
     bp.goff.assign(ng, 0);

@@ -51,6 +51,37 @@ __device__ __forceinline__ unsigned long long warp_max(unsigned long long v)
     return ((unsigned long long) mhi << 32) | mlo;
 }
 
+// Two floats in one 64-bit register and the packed operations of sm_100 on them:
+// each half is rounded to nearest as the scalar operation (no flush to zero), so
+// `sub2(sub2(fma2(a, b, nz), c), d)` gives per half the bits of
+// __fsub_rn(__fsub_rn(__fmul_rn(a, b), c), d) with half the issues. The product is
+// a fused operation with the addend -0, which changes no product, handed to the
+// kernel as an argument: mul.rn.f32x2 followed by sub.rn.f32x2 is compiled into one
+// fused operation (nine in ten of random operands gave its bits on the device), and
+// a constant -0 would let the compiler see the product.
+__device__ __forceinline__ unsigned long long f2(float a, float b)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_split(unsigned long long v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 

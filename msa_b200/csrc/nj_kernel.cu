@@ -60,32 +60,6 @@ constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
 // Row chunks (4 floats) each lane has in flight while scanning.
 constexpr int kBatch = 4;
-// Two float lanes in one 64-bit register and the packed float operations of
-// sm_100 on them: each lane is rounded to nearest as the scalar operation
-// (no flush to zero), so `sub2(sub2(mul2(a, b), c), d)` gives per lane the
-// bits of __fsub_rn(__fsub_rn(__fmul_rn(a, b), c), d) with half the issues.
-__device__ __forceinline__ unsigned long long f2(float a, float b)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void f2_split(unsigned long long v, float &a, float &b)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b)
-{
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b)
-{
-    unsigned long long r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 
 struct State {
     float *D;                  // n rows of P floats; slot t + k holds logical k
@@ -107,6 +81,7 @@ struct State {
     uint32_t *cand_seq;        // [helper_ctas] join number + 1 of its last candidate
     unsigned long long wait_ns;   // limit of every wait between clusters
     int stall_publication;     // test hook: the folding CTA never publishes
+    float nz;                  // -0 (see fma2)
 };
 
 constexpr uint32_t kStop = 0xffffffffu;
@@ -170,7 +145,7 @@ struct ScanView {
     const float *D;   // slot t + k holds logical k; row pitch P
     const float *S;   // this CTA's row sums by slot
     uint32_t P, t, c, pend, moved, mslot;
-    float cm2, s_moved;
+    float cm2, s_moved, nz;
 };
 
 template <bool TailCut>
@@ -180,15 +155,15 @@ __device__ __forceinline__ void scan_rows(const ScanView &v, uint32_t s, uint32_
     const uint32_t W = ns * kWarps, gw = (uint32_t) warp * ns + s;
     const uint32_t base4 = v.t & ~3u;
     const float s_moved = v.s_moved;
-    const unsigned long long cm2x2 = f2(v.cm2, v.cm2);
+    const unsigned long long cm2x2 = f2(v.cm2, v.cm2), nz2 = f2(v.nz, v.nz);
     auto row_of = [&](uint32_t i) { return v.D + (size_t) (i == v.moved ? v.mslot : v.t + i) * v.P + base4; };
     // Q = (c-2) * D - S_i - S_j for the four cells of a chunk, two per packed
     // operation; cells at or past the row's end (column hi) get -inf.
     auto chunk_raw = [&](const float4 &d, uint32_t col, unsigned long long si2, float &q0, float &q1, float &q2,
                          float &q3) {
         const float4 s = *reinterpret_cast<const float4 *>(v.S + col);
-        f2_split(sub2(sub2(mul2(cm2x2, f2(d.x, d.y)), si2), f2(s.x, s.y)), q0, q1);
-        f2_split(sub2(sub2(mul2(cm2x2, f2(d.z, d.w)), si2), f2(s.z, s.w)), q2, q3);
+        f2_split(sub2(sub2(fma2(cm2x2, f2(d.x, d.y), nz2), si2), f2(s.x, s.y)), q0, q1);
+        f2_split(sub2(sub2(fma2(cm2x2, f2(d.z, d.w), nz2), si2), f2(s.z, s.w)), q2, q3);
     };
     auto chunk_q = [&](const float4 &d, uint32_t col, uint32_t hi, unsigned long long si2, float &q0, float &q1,
                        float &q2, float &q3) {
@@ -333,7 +308,7 @@ __device__ void nj_helper(const State &st, float *S, uint32_t hidx, uint32_t sid
     uint32_t c = n, t = 0, step = 0, pend = kNone, moved = kNone, mslot = 0;
     while(c > 1 && c > st.helper_c) {
         unsigned long long best = 0;
-        scan_rows<!Linear>(ScanView{st.D, S, P, t, c, pend, moved, mslot, (float) (c - 2), h_moved}, sidx, nscan, warp,
+        scan_rows<!Linear>(ScanView{st.D, S, P, t, c, pend, moved, mslot, (float) (c - 2), h_moved, st.nz}, sidx, nscan, warp,
                            lane,
                   best);
         {
@@ -485,7 +460,7 @@ __global__ void __launch_bounds__(kThreads, 1) nj_cluster_kernel(State st)
             // This CTA's share of the rows of the logical lower triangle
             // (scan_rows), with +inf in S masking the dropped slots and those
             // of `moved` and the new node.
-            scan_rows<!Linear>(ScanView{D, S, P, t, c, pend, moved, mslot, cm2, s_moved_sh}, rank,
+            scan_rows<!Linear>(ScanView{D, S, P, t, c, pend, moved, mslot, cm2, s_moved_sh, st.nz}, rank,
                       F + (helped ? st.helper_ctas : 0u), warp, lane, best);
         } else if(pend != kNone) {
             // The new node's row and column, from the distances the last join
@@ -989,6 +964,7 @@ int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, msa_o
         st.cand = (unsigned long long *) (base + oCand);
         st.wait_ns = (unsigned long long) (ctx->nj_wait_us ? ctx->nj_wait_us : kWaitUs) * 1000ull;
         st.stall_publication = ctx->nj_stall;
+        st.nz = -0.0f;
         MSA_CUDA_TRY(ctx, cudaMemsetAsync(sync, 0, 64 + (size_t) kMaxHelperCtas * 4, s));
         MSA_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[1], s));
         MSA_CUDA_TRY(ctx, launch_clusters(kern_help, K, K * clusters, kThreads, help_smem, s, st));

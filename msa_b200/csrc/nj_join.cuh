@@ -29,8 +29,9 @@
 // a bound, so the first search of a launch reads the whole matrix. Any
 // non-finite or huge value switches the bounds off and every row is scanned
 // every time. On matrices of related, of independent and of very uneven
-// sequences 14 to 28 rows of 2,000 to 5,000 are read per join, and 150 where
-// only four distinct scores make most pairs tie.
+// sequences 14 to 28 rows of 2,000 to 5,000 are read per join, 158 where only four
+// distinct scores make many pairs tie, and all of them among copies of one sequence;
+// there the launch gives up (kManyRows).
 //
 // Phases of a join:
 //   search  every CTA owns the rows of slots = rank mod K: it scans those whose
@@ -52,12 +53,11 @@
 //
 // Measured beside a search of the whole lower triangle at every join (one
 // cluster of 16 CTAs, slices of the join exchanged over a second barrier):
-// 5,000 proteins 90.6 -> 43.9 ms, 2,000 proteins 15.2 -> 11.4 ms (the 2,000-taxon
-// pipeline matrix 14.9 -> 11.2), 257 proteins 1.34 -> 0.82 ms with its upload,
-// 120 proteins 0.55 -> 0.25 ms. What bounds a join now is the latency of its
-// phases, not the matrix: at 2,000 nodes about 3,900 cycles for the rows
-// scanned (the fold beside them 3,600), 1,800 to take in the new node, 1,800
-// to the barrier and across it, 3,500 for the join.
+// 5,000 proteins 90.6 -> 38.3 ms, 2,000 proteins 15.2 -> 10.0 ms, 257 proteins
+// 1.34 -> 0.76 ms with its upload, 120 proteins 0.55 -> 0.23 ms. What bounds a join
+// now is the latency of its phases, not the matrix: at 2,000 nodes about 3,600 cycles
+// for the rows scanned (the fold beside them 3,300), 1,500 to take in the new node,
+// 1,900 to the barrier and across it, 2,900 for the join.
 #pragma once
 
 #include "nj_device.cuh"
@@ -72,6 +72,13 @@ constexpr int kFoldWarps = 2;                   // fold a row sum while the othe
 constexpr int kScanWarps = kJoinWarps - kFoldWarps;
 constexpr int kFoldParts = kFoldWarps * 8;      // four lanes each
 constexpr uint32_t kDead = 0xffffu;             // pos of a slot without a live node; no partner
+// Where copies of a sequence or few distinct scores make many pairs tie, every row
+// that ties is read at every join, and a search of every pair (nj_cluster_kernel,
+// on a matrix that holds the live nodes alone) is quicker. A CTA's rows beyond
+// `rows_allowed` are added up over the joins; where they come to kExcessJoins joins'
+// worth, the launch ends with kManyRows and the host goes on with that kernel.
+constexpr int kManyRows = 5, kExcessJoins = 16;
+constexpr uint32_t kGiveUp = 0x80000000u;   // in a candidate's slots, which take 14 bits each
 // Float4 loads each lane keeps in flight while it scans a row.
 constexpr int kRowBatch = 4;
 constexpr size_t kMaxSmem = 227 * 1024 - 4096;   // dynamic, beside up to 4 KB of static shared memory
@@ -85,7 +92,9 @@ struct Stage {
     uint32_t *mabs;            // bits of the largest |D| so far (above 0x7f7fffff: not finite)
     uint32_t *rec_x, *rec_y;   // logical indices joined at each step
     float *rec_dx, *rec_dy;
-    int *err;                  // 2: no joinable pair; 4: an invalid pair
+    int *err;                  // 2: no joinable pair; 4: an invalid pair; kManyRows
+    uint32_t *left;            // kManyRows: nodes of the launch that gave up, and those it left
+    uint32_t rows_allowed;     // rows per join and CTA beyond which the launch gives up (0: any number)
     unsigned long long *cycles;
     uint32_t N, P, c_end, step0;
     // nj_small_kernel only: the packed triangle (float, or int32 converted
@@ -288,18 +297,13 @@ __device__ __forceinline__ Cand shfl_cand(const Cand &c, int src)
                 __shfl_sync(kFull, c.order, src)};
 }
 
+// Of two pairs of one node, the reference's row-major scan meets the one with the
+// smaller logical partner first: partners below the node are columns of its row,
+// those above it are rows further down.
 struct RowScan {
     float m1, m2, d1, dmin;   // best Q, best of the others, D of the best, smallest D
     uint32_t j1;
 };
-
-// (i, j) before (i, k) in the reference's row-major order, from the logical
-// indices a of j, b of k and pi of i.
-__device__ __forceinline__ bool pair_before(uint32_t a, uint32_t b, uint32_t pi)
-{
-    const uint32_t ja = max(a, pi), jb = min(a, pi), ka = max(b, pi), kb = min(b, pi);
-    return ja < ka || (ja == ka && jb < kb);
-}
 
 // Q of the pair (i, j): the row sum of the logically later node is subtracted
 // first, as the reference does.
@@ -311,8 +315,7 @@ __device__ __forceinline__ float pair_q(float cm2, float d, float si, uint32_t p
 
 // A row scanned by `wpr` warps of which this is number `sub`: the lane's two
 // largest Q, the pair of the first and the smallest distance. The loop holds
-// no branch; equal Q show as m2 == m1, and only then are the lane's cells
-// gone through again for the first pair in the reference's order.
+// no branch; equal Q show as m2 == m1 (see merge_row).
 __device__ __forceinline__ RowScan scan_row(const float *__restrict__ row, const float *S, const uint16_t *pos,
                                             uint32_t i, uint32_t P, float cm2, uint32_t sub, uint32_t wpr, int lane)
 {
@@ -349,27 +352,11 @@ __device__ __forceinline__ RowScan scan_row(const float *__restrict__ row, const
             }
         }
     }
-    if(r.m1 == r.m2 && r.j1 != kDead) {
-        uint32_t first = pos[r.j1];
-#pragma unroll 1
-        for(uint32_t g = sub * 32 + lane; g < nch; g += stride)
-#pragma unroll 1
-            for(uint32_t j = 4 * g; j < 4 * g + 4; ++j) {
-                const uint32_t pj = pos[j];
-                if(S[j] == INFINITY || pj == pi) continue;
-                const float d = __ldcg(row + j);
-                if(pair_q(cm2, d, si, pi, S[j], pj) == r.m1 && pair_before(pj, first, pi)) {
-                    first = pj;
-                    r.j1 = j;
-                    r.d1 = d;
-                }
-            }
-    }
     return r;
 }
 
-// The lanes' scans of one row (logical index pi) as one; every lane gets it.
-__device__ __noinline__ RowScan merge_scans(const RowScan &r, const uint16_t *pos, uint32_t pi, int lane)
+// The lanes' scans of one row as one; every lane gets it.
+__device__ __forceinline__ RowScan merge_scans(const RowScan &r, const uint16_t *pos, int lane)
 {
     RowScan o;
     o.m1 = warp_fmax(r.m1);
@@ -377,10 +364,9 @@ __device__ __noinline__ RowScan merge_scans(const RowScan &r, const uint16_t *po
     uint32_t who = __ballot_sync(kFull, r.m1 == o.m1 && r.j1 != kDead);
     if(__popc(who) > 1) {   // equal Q: the first pair in the reference's order
         const bool in = (who >> lane) & 1u;
-        const uint32_t pj = in ? pos[r.j1] : 0u;
-        const uint32_t order = in ? max(pj, pi) << 16 | min(pj, pi) : 0xffffffffu;
-        const uint32_t first = __reduce_min_sync(kFull, order);
-        who = __ballot_sync(kFull, in && order == first);
+        const uint32_t pj = in ? pos[r.j1] : kDead;
+        const uint32_t first = __reduce_min_sync(kFull, pj);
+        who = __ballot_sync(kFull, pj == first);
     }
     const int src = who ? __ffs(who) - 1 : 0;
     o.m2 = warp_fmax(who && lane == src ? r.m2 : r.m1);
@@ -388,6 +374,47 @@ __device__ __noinline__ RowScan merge_scans(const RowScan &r, const uint16_t *po
     o.j1 = __shfl_sync(kFull, r.j1, src);
     if(who == 0u) o.j1 = kDead;
     return o;
+}
+
+// The same after a scan of the row: lanes with several cells of the row's largest Q
+// go through their cells again, with the scan's loads, for the first of them (2,000
+// nodes, a quarter of them copies of one: 17.6 ms with one load at a time, 10.6 so).
+__device__ __noinline__ RowScan merge_row(RowScan r, const float *__restrict__ row, const float *S,
+                                          const uint16_t *pos, uint32_t i, uint32_t P, float cm2, uint32_t sub,
+                                          uint32_t wpr, int lane)
+{
+    const float top = warp_fmax(r.m1);
+    if(r.m1 == r.m2 && r.m1 == top && r.j1 != kDead) {
+        const float si = S[i];
+        const uint32_t pi = pos[i], nch = P >> 2, stride = 32 * wpr;
+        uint32_t first = pos[r.j1];
+#pragma unroll 1
+        for(uint32_t g0 = sub * 32 + lane; g0 < nch; g0 += kRowBatch * stride) {
+            float4 d[kRowBatch];
+#pragma unroll
+            for(int u = 0; u < kRowBatch; ++u)
+                if(g0 + u * stride < nch) d[u] = __ldcg(reinterpret_cast<const float4 *>(row) + g0 + u * stride);
+#pragma unroll
+            for(int u = 0; u < kRowBatch; ++u) {
+                const uint32_t g = g0 + u * stride;
+                if(g >= nch) break;
+                const float4 s4 = *reinterpret_cast<const float4 *>(S + 4 * g);
+                const uint2 p4 = *reinterpret_cast<const uint2 *>(pos + 4 * g);
+                const float dd[4] = {d[u].x, d[u].y, d[u].z, d[u].w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
+                const uint32_t pp[4] = {p4.x & 0xffffu, p4.x >> 16, p4.y & 0xffffu, p4.y >> 16};
+#pragma unroll
+                for(int k = 0; k < 4; ++k)
+                    if(pp[k] < first && pp[k] != pi && ss[k] != INFINITY &&
+                       pair_q(cm2, dd[k], si, pi, ss[k], pp[k]) == r.m1) {
+                        first = pp[k];
+                        r.j1 = 4 * g + k;
+                        r.d1 = dd[k];
+                    }
+            }
+        }
+    }
+    __syncwarp();
+    return merge_scans(r, pos, lane);
 }
 
 template <bool Linear>
@@ -420,6 +447,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
     __shared__ float sz_sh;
     __shared__ Joined joined;
     __shared__ uint32_t nlist;
+    __shared__ int excess;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if(*st.err != 0) return;   // an earlier launch failed (the same for every CTA)
@@ -441,6 +469,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
     if(tid < 2 * (int) kMaxCluster) parts[tid / kMaxCluster][tid % kMaxCluster] = no_cand();
     if(tid == 0) {
         nlist = 0;
+        excess = 0;
         sz_sh = 0.0f;
     }
     uint32_t sv = size_of(__uint_as_float(*st.mabs), 0.0f);
@@ -510,7 +539,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
             float L = -INFINITY;
             {
                 const Cand v = lane < 16 ? wcand[lane] : parts[(step - 1) & 1u][lane - 16];
-                const uint32_t i = v.slots >> 16, j = v.slots & 0xffffu;
+                const uint32_t i = v.slots >> 16 & 0x7fffu, j = v.slots & 0xffffu;
                 if(v.q > -INFINITY && i != z && j != z) {
                     const uint32_t pi = pos[i], pj = pos[j];
                     if(pi != kDead && pj != kDead) L = q_of(pi, S[i], pj, S[j], v.d);
@@ -543,8 +572,9 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
 #pragma unroll 1
             for(uint32_t k = w >> lg; k < m; k += rows) {   // once where warps share a row: m <= rows
                 const uint32_t l = list[k], i = l * K + rank;
-                const RowScan o = merge_scans(
-                    scan_row(D + (size_t) i * P, S, pos, i, P, cm2, w & (wpr - 1), wpr, lane), pos, pos[i], lane);
+                const float *row = D + (size_t) i * P;
+                const RowScan o = merge_row(scan_row(row, S, pos, i, P, cm2, w & (wpr - 1), wpr, lane), row, S, pos, i,
+                                            P, cm2, w & (wpr - 1), wpr, lane);
                 if(wpr > 1) {
                     if(lane == 0) wscan[w] = o;
                 } else {
@@ -554,10 +584,10 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
             if(wpr > 1) {
                 scan_sync();
                 if(w < m) {
-                    const uint32_t l = list[w], i = l * K + rank;
+                    const uint32_t l = list[w];
                     RowScan r{-INFINITY, -INFINITY, 0.0f, 3.0e38f, kDead};
                     if((uint32_t) lane < wpr) r = wscan[(w << lg) + lane];
-                    renew(l, merge_scans(r, pos, pos[i], lane));
+                    renew(l, merge_scans(r, pos, lane));
                 }
             }
             mark(cyc_scan);
@@ -570,6 +600,8 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
             const uint32_t pz = z != kDead ? pos[z] : kDead;
             if(tid == 0) {
                 if(z != kDead) S[z] = sz;   // read again only after the next barrier
+                // Rows read beyond the allowance of each join (the first one reads all).
+                if(step > 0) excess = max(excess + (int) nlist - (int) st.rows_allowed, 0);
                 nlist = 0;
             }
             Cand best = no_cand();
@@ -586,7 +618,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
                 }
                 if(z != kDead) {
                     const float dz = ND[l], qz = q_of(pi, si, pz, sz, dz);
-                    const bool take = qz > q || (qz == q && pair_before(pz, pj, pi));
+                    const bool take = qz > q || (qz == q && pz < pj);
                     const float B = bound(l, si), other = __fadd_ru(take ? q : qz, slack);
                     if(other > B || dz < Dm[l]) {
                         Dm[l] = fminf(Dm[l], dz);
@@ -611,7 +643,8 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
         const uint32_t buf = step & 1u;
         if(warp == 0) {
             const Cand v = lane < kJoinWarps ? wcand[lane] : no_cand();
-            const Cand o = shfl_cand(v, best_lane(v, lane));
+            Cand o = shfl_cand(v, best_lane(v, lane));
+            if(st.rows_allowed != 0 && excess > kExcessJoins * (int) st.rows_allowed) o.slots |= kGiveUp;
             if((uint32_t) lane < K) *cluster.map_shared_rank(&parts[buf][rank], (unsigned) lane) = o;
         }
         mark(cyc_new);
@@ -621,7 +654,9 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
 
         // ---- join
         Cand win = (uint32_t) lane < K ? parts[buf][lane] : no_cand();
+        const bool give_up = __any_sync(kFull, (win.slots & kGiveUp) != 0u);
         win = shfl_cand(win, best_lane(win, lane));
+        win.slots &= ~kGiveUp;
         if(win.q == -INFINITY) {   // no selectable Q (all NaN): the reference would index an undefined pair
             failed = true;
             break;
@@ -728,10 +763,16 @@ __global__ void __launch_bounds__(kJoinThreads, 1) nj_join_kernel(Stage st)
         ++step;
         --c;
         mark(cyc_join);
+        if(give_up) break;
     }
     if(rank == 0 && tid == 0) {
         if(failed) atomicExch(st.err, 2);
         if(bad) atomicExch(st.err, 4);
+        if(!failed && !bad && c > st.c_end) {
+            st.left[0] = N;
+            st.left[1] = c;
+            atomicExch(st.err, kManyRows);
+        }
     }
     if(rank == 0) {
         if(!failed && !bad) {

@@ -3,9 +3,12 @@
 // njoining::sequential<transform::linear<2>>
 // (src/phylogeny/njoining/impl/sequential.cpp:80-358).
 //
-// nj_join.cuh holds the kernels that a run uses; nj_cluster_kernel below is the
-// one that can spread a join's search over more clusters (msa_nj_set_clusters),
-// and runs only when the context asks for that.
+// nj_join.cuh holds the kernels that a run starts with; nj_cluster_kernel below
+// searches every pair at every join. It runs where most rows would be read anyway
+// (many pairs tie: a launch of nj_join_kernel gives up and it takes over), where no
+// cluster can hold the row states of nj_join_kernel (many nodes, clusters of fewer
+// than 16 CTAs), and where the context spreads a join's search over several clusters
+// (msa_nj_set_clusters).
 //
 // Layout. The reference keeps a packed symmetric matrix and, after every join,
 // swaps the removed OTU y with logical 0 and deletes logical 0
@@ -850,9 +853,22 @@ constexpr uint32_t kTinyNodes = 64;
 // too, and each packing costs one search of the whole smaller matrix.
 constexpr double kStageShare = 0.6;
 
+// Rows that a CTA of a launch of N nodes may read per join before a search of every
+// pair is the better one (0: it never is). A CTA reads 14 rows at a time, in a time
+// that grows with N, while a search of every pair grows with its square. 2,000 nodes,
+// going on against giving up: 16.0 and 15.3 ms at 9 rows per CTA and join (two
+// distinct distances), 17.1 and 15.6 at 10 (four), 29 and 15.8 at 31 (eleven), 65 and
+// 14.9 at 70 (one); 12.0 and over 15 at 4. 700 nodes: 3.2 and 3.7 at 6, 5.8 and 3.4
+// at 29. 300 nodes: 1.1 and 1.4 with every row read.
+uint32_t rows_allowed(uint32_t N)
+{
+    return N < 512 ? 0 : std::max(8u, N / 200);
+}
+
 }  // namespace njdev
 
-int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, msa_otu *out)
+// `bounded`: whether launches that read many rows give up (Stage::rows_allowed).
+static int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, bool bounded, msa_otu *out)
 {
     using namespace njdev;
     const bool linear = order == MSA_NJ_LINEAR;
@@ -918,6 +934,7 @@ int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, msa_o
     unsigned long long *d_cycles = (unsigned long long *) (base + oHead);
     int *d_err = (int *) (base + oHead + 64);
     uint32_t *d_mabs = (uint32_t *) (base + oHead + 68);
+    uint32_t *d_left = (uint32_t *) (base + oHead + 72);
     uint32_t *rec = (uint32_t *) (base + oRec);
     float *rec_f = (float *) (base + oRec);
 
@@ -942,18 +959,19 @@ int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, msa_o
         ctx->launches += 2;
     }
 
-    if(helped) {
+    // All joins of `m` nodes by the kernel that searches every pair.
+    auto search_all = [&](float *D, const float *S, uint32_t m) {
         State st{};
-        st.D = (float *) (base + oD);
-        st.S0 = (const float *) (base + oS);
-        st.rec_x = rec;
-        st.rec_y = rec + n;
-        st.rec_dx = rec_f + 2 * (size_t) n;
-        st.rec_dy = rec_f + 3 * (size_t) n;
+        st.D = D;
+        st.S0 = S;
+        st.rec_x = rec + (n - m);
+        st.rec_y = rec + n + (n - m);
+        st.rec_dx = rec_f + 2 * (size_t) n + (n - m);
+        st.rec_dy = rec_f + 3 * (size_t) n + (n - m);
         st.err = d_err;
         st.cycles = d_cycles;
-        st.n = n;
-        st.P = P;
+        st.n = m;
+        st.P = pitch(m);
         char *sync = base + oSync;
         st.helper_ctas = (clusters - 1) * K;
         st.helper_c = helper_c;
@@ -965,9 +983,12 @@ int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, msa_o
         st.wait_ns = (unsigned long long) (ctx->nj_wait_us ? ctx->nj_wait_us : kWaitUs) * 1000ull;
         st.stall_publication = ctx->nj_stall;
         st.nz = -0.0f;
-        MSA_CUDA_TRY(ctx, cudaMemsetAsync(sync, 0, 64 + (size_t) kMaxHelperCtas * 4, s));
+        return launch_clusters(kern_help, K, K * clusters, kThreads, (size_t) st.P * 16, s, st);
+    };
+    if(helped) {
+        MSA_CUDA_TRY(ctx, cudaMemsetAsync(base + oSync, 0, 64 + (size_t) kMaxHelperCtas * 4, s));
         MSA_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[1], s));
-        MSA_CUDA_TRY(ctx, launch_clusters(kern_help, K, K * clusters, kThreads, help_smem, s, st));
+        MSA_CUDA_TRY(ctx, search_all((float *) (base + oD), (const float *) (base + oS), n));
         ctx->launches++;
     } else {
         MSA_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[1], s));
@@ -990,6 +1011,8 @@ int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, msa_o
             st.rec_dx = rec_f + 2 * (size_t) n;
             st.rec_dy = rec_f + 3 * (size_t) n;
             st.err = d_err;
+            st.left = d_left;
+            st.rows_allowed = bounded ? rows_allowed(st.N) : 0;
             st.cycles = d_cycles;
             st.tri = direct ? dtri : nullptr;
             st.tri_int = is_int;
@@ -1025,6 +1048,31 @@ int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, msa_o
     int err = 0;
     std::memcpy(cyc, back.data(), sizeof(cyc));
     std::memcpy(&err, back.data() + 16, sizeof(err));
+    if(err == kManyRows) {
+        // The live nodes of the launch that gave up, packed, and the other kernel.
+        const uint32_t N = back[18], m = back[19];
+        const bool odd = (std::find(stages.begin(), stages.end(), N) - stages.begin()) & 1;
+        int resident = 0;
+        K = pick_cluster(kern_help, kThreads, [&](unsigned) { return (size_t) pitch(m) * 16; }, &resident);
+        void *D = nullptr;
+        size_t bytes = 0;
+        if(K < 2 || ctx->blocks.take((size_t) (m + 1) * pitch(m) * 4, &D, &bytes))
+            return nj_run(ctx, tri, kind, n, order, false, out);
+        cudaError_t e = cudaMemsetAsync(d_err, 0, 4, s);
+        compact_kernel<<<std::min<uint32_t>(m + 1, 4 * (uint32_t) ctx->num_sms), 256, 0, s>>>(
+            (const float *) (base + (odd ? oD2 : oD)), pitch(N), (const uint32_t *) (base + oOrd), (float *) D, m, pitch(m),
+            d_err);
+        if(!e) e = cudaGetLastError();
+        if(!e) e = search_all((float *) D, (const float *) (base + (odd ? oS : oS2)), m);
+        ctx->launches += 2;
+        if(!e) e = cudaEventRecord(ctx->ev[2], s);
+        if(!e) e = cudaMemcpyAsync(back.data(), base + oHead, back.size() * 4, cudaMemcpyDeviceToHost, s);
+        const cudaError_t done = cudaStreamSynchronize(s);
+        ctx->blocks.give(D, bytes);
+        MSA_CUDA_TRY(ctx, e ? e : done);
+        std::memcpy(cyc, back.data(), sizeof(cyc));
+        std::memcpy(&err, back.data() + 16, sizeof(err));
+    }
     {
         msa_nj_stats ns{};
         float ms = 0, ms_all = 0;
@@ -1094,6 +1142,11 @@ int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, msa_o
         out[parent].child[1] = c2;
     }
     return MSA_OK;
+}
+
+int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, msa_otu *out)
+{
+    return nj_run(ctx, tri, kind, n, order, true, out);
 }
 
 }  // namespace msa

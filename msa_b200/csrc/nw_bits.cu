@@ -78,13 +78,10 @@ __device__ __forceinline__ int count_bits(uint32_t x, int lane)
     return __popc(x);
 }
 
-// One task. `ring`: the warp's kRingRows rows of S words. S is 0 mod 32 where the lanes are on 32 different columns, and
-// 8 or 16 where 4 or 2 lanes are on one: equal columns of the first letters
-// then lie in different banks.
-// Progress of the warps of a CTA that share a task's strips (null: one warp has
-// all of them): (strip + 1) << 16 | columns of its last row that may be read.
+// Progress of the warps of a CTA that share a task's strips, as strip_progress gives
+// it (null: one warp has all of them).
 struct Strips {
-    volatile uint32_t *done;
+    volatile unsigned long long *done;
     int *err;
 };
 // A strip waits at most this long for the one above it.
@@ -92,7 +89,7 @@ constexpr unsigned long long kStripWaitNs = 5000000000ull;
 
 // Waits until *done >= want, or gives up: then, and in every later wait of the
 // launch, the strip runs on with what is there and the call fails.
-__device__ __noinline__ void strip_wait(volatile uint32_t *done, uint32_t want, int *err)
+__device__ __noinline__ void strip_wait(volatile unsigned long long *done, unsigned long long want, int *err)
 {
     unsigned long long t0, t1;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
@@ -107,6 +104,9 @@ __device__ __noinline__ void strip_wait(volatile uint32_t *done, uint32_t want, 
     }
 }
 
+// One task. `ring`: the warp's kRingRows rows of S words. S is 0 mod 32 where the
+// lanes are on 32 different columns, and 8 or 16 where 4 or 2 lanes are on one: equal
+// columns of the first letters then lie in different banks.
 template <int R, int LP>
 __device__ __noinline__ void bit_task(const BitParams &p, const BitSet &set, uint32_t grp, uint32_t *ring,
                                       uint2 *bound, int lane, int s0 = 0, int ds = 1, const Strips &strips = Strips{nullptr, nullptr})
@@ -170,10 +170,10 @@ __device__ __noinline__ void bit_task(const BitParams &p, const BitSet &set, uin
                 // Lane 31 has stored the columns up to c0 - 32.
                 if(lane == 31 && c0 > 31) {
                     __threadfence_block();
-                    strips.done[st % ds] = (uint32_t) (st + 1) << 16 | (uint32_t) (c0 - 31);
+                    strips.done[st % ds] = strip_progress((uint32_t) st, (uint32_t) (c0 - 31));
                 }
                 if(st > 0) {
-                    const uint32_t want = (uint32_t) st << 16 | (uint32_t) min(c0 + 32, ncols);
+                    const unsigned long long want = strip_progress((uint32_t) st - 1, (uint32_t) min(c0 + 32, ncols));
                     if(strips.done[(st - 1) % ds] < want) strip_wait(strips.done + (st - 1) % ds, want, strips.err);
                     __threadfence_block();
                 }
@@ -221,7 +221,7 @@ __device__ __noinline__ void bit_task(const BitParams &p, const BitSet &set, uin
         __syncwarp();
         if(LP == 32 && strips.done && lane == 31) {
             __threadfence_block();
-            strips.done[st % ds] = (uint32_t) (st + 1) << 16 | 0xffffu;
+            strips.done[st % ds] = strip_progress((uint32_t) st, 0xffffffffu);
         }
     }
     if((nst - 1) % ds != s0) return;   // another warp has the last row
@@ -306,7 +306,7 @@ constexpr size_t kRingBytes = kBitWarps * kRingWords * sizeof(uint32_t);
 __global__ void __launch_bounds__(kBitWarps * 32, 4) nw_bits_kernel(BitParams p)
 {
     extern __shared__ __align__(16) uint32_t rings[];
-    __shared__ uint32_t done[kBitWarps];
+    __shared__ unsigned long long done[kBitWarps];
     __shared__ unsigned long long task;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t *ring = rings + warp * kRingWords;

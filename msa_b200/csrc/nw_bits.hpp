@@ -44,6 +44,14 @@ constexpr int kBitWarps = 4;   // per CTA
 // Longest columns: the sums of one lane's columns take 12 bits.
 constexpr uint32_t kBitMaxCols = 40000;
 
+// Progress of a chained set: `columns` columns of the last row of strip `strip` may be
+// read. The word of any later strip is greater than every word of an earlier one: a
+// sequence of 2^30 units has more than 2^20 strips.
+__host__ __device__ constexpr unsigned long long strip_progress(uint32_t strip, uint32_t columns)
+{
+    return (unsigned long long) (strip + 1) << 32 | columns;
+}
+
 __host__ __device__ __forceinline__ uint32_t bit_pitch(uint32_t ncols) { return (ncols + 31) / 32 * 32 + 64; }
 __host__ __device__ __forceinline__ uint32_t bit_bound(uint32_t ncols) { return (ncols + 31) / 32 * 32 + 96; }
 

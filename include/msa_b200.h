@@ -194,6 +194,13 @@ int msa_nw_part_of_pairs(const uint8_t *units, const uint64_t *offs, const uint6
  * in the reference (its one kernel shape is fixed, hybrid.cu:57). */
 int msa_nw_set_tiles(msa_ctx *ctx, int rows_per_lane, int warps_per_cta);
 
+/* Limit of the waits between the strips of a long sequence that run on several
+ * warps or CTAs (no counterpart in the reference); 0 = the default, 5 s. A wait
+ * that runs out fails the call with MSA_ERR_DEVICE_TIMEOUT and leaves the
+ * context and the store usable (a limit of 1 us makes some run out wherever
+ * strips wait at all). Applies to later calls. */
+int msa_nw_set_wait(msa_ctx *ctx, uint32_t wait_limit_us);
+
 /* Variants of the persistent kernel, for measuring what each of its parts
  * contributes (no counterpart in the reference, which has one kernel). Flags:
  * MSA_NW_VARIANT_INT32 runs every task in 32-bit lanes (one rows sequence at

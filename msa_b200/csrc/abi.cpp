@@ -487,6 +487,13 @@ int msa_nw_set_tiles(msa_ctx *ctx, int rows_per_lane, int warps_per_cta)
     return MSA_OK;
 }
 
+int msa_nw_set_wait(msa_ctx *ctx, uint32_t wait_limit_us)
+{
+    if(!ctx) return MSA_ERR_INVALID;
+    ctx->nw_wait_us = wait_limit_us;
+    return MSA_OK;
+}
+
 int msa_nw_last_stats(const msa_ctx *ctx, msa_nw_stats *out)
 {
     if(!ctx || !out) return MSA_ERR_INVALID;

@@ -83,20 +83,20 @@ __device__ __forceinline__ int count_bits(uint32_t x, int lane)
 struct Strips {
     volatile unsigned long long *done;
     int *err;
+    unsigned long long wait_ns;   // limit of a strip's wait for the one above it
 };
-// A strip waits at most this long for the one above it.
-constexpr unsigned long long kStripWaitNs = 5000000000ull;
 
 // Waits until *done >= want, or gives up: then, and in every later wait of the
 // launch, the strip runs on with what is there and the call fails.
-__device__ __noinline__ void strip_wait(volatile unsigned long long *done, unsigned long long want, int *err)
+__device__ __noinline__ void strip_wait(volatile unsigned long long *done, unsigned long long want, int *err,
+                                        unsigned long long wait_ns)
 {
     unsigned long long t0, t1;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
     while(*done < want) {
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
         if(*(volatile int *) err != 0) break;
-        if(t1 - t0 > kStripWaitNs) {
+        if(t1 - t0 > wait_ns) {
             atomicExch(err, 1);
             break;
         }
@@ -109,7 +109,8 @@ __device__ __noinline__ void strip_wait(volatile unsigned long long *done, unsig
 // columns of the first letters then lie in different banks.
 template <int R, int LP>
 __device__ __noinline__ void bit_task(const BitParams &p, const BitSet &set, uint32_t grp, uint32_t *ring,
-                                      uint2 *bound, int lane, int s0 = 0, int ds = 1, const Strips &strips = Strips{nullptr, nullptr})
+                                      uint2 *bound, int lane, int s0 = 0, int ds = 1,
+                                      const Strips &strips = Strips{nullptr, nullptr, 0})
 {
     constexpr int S = 96 + (LP == 8 ? 8 : LP == 16 ? 16 : 0), U = R <= 8 ? 4 : R <= 16 ? 2 : 1;
     const int at = lane % LP, ncols = (int) p.gcols[grp];
@@ -174,7 +175,8 @@ __device__ __noinline__ void bit_task(const BitParams &p, const BitSet &set, uin
                 }
                 if(st > 0) {
                     const unsigned long long want = strip_progress((uint32_t) st - 1, (uint32_t) min(c0 + 32, ncols));
-                    if(strips.done[(st - 1) % ds] < want) strip_wait(strips.done + (st - 1) % ds, want, strips.err);
+                    if(strips.done[(st - 1) % ds] < want)
+                        strip_wait(strips.done + (st - 1) % ds, want, strips.err, strips.wait_ns);
                     __threadfence_block();
                 }
                 __syncwarp();
@@ -330,7 +332,7 @@ __global__ void __launch_bounds__(kBitWarps * 32, 4) nw_bits_kernel(BitParams p)
         const BitSet set = find((uint32_t) q);
         const uint32_t grp = max(p.g0, set.a / 32) + (uint32_t) q - set.first;
         uint2 *bound = p.bound + blockIdx.x * kBitWarps * p.bound_words;
-        const dev::Strips strips{done, p.err};
+        const dev::Strips strips{done, p.err, p.wait_ns};
 #define MSA_BITS(RR) case RR: dev::bit_task<RR, 32>(p, set, grp, ring, bound, lane, warp, kBitWarps, strips); break;
         if(warp < (int) set.nst)
             switch(set.R) {

@@ -33,6 +33,7 @@ struct BitParams {
     uint32_t nchain;                // tasks of the first sets, taken by whole CTAs
     int *err;                       // set when a wait between strips ran out
     unsigned long long *counter;    // of chained tasks, and of the others
+    unsigned long long wait_ns;     // limit of the waits between strips
 };
 
 // Rows of match words: the letters, and which columns lie within a sequence.

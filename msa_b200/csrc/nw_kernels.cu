@@ -365,8 +365,9 @@ constexpr uint8_t kRowNarrow = 1, kRowQuad = 2, kRowLong = 4, kRowChain = 8, kRo
 constexpr int kRebase = 512;
 // Columns between two publications of a chained strip's progress.
 constexpr int kPublish = 64;
-// A chained strip waits at most this long for the one above it.
-constexpr unsigned long long kChainWaitNs = 5000000000ull;
+// A chained strip waits at most this long for the one above it, unless the context
+// says otherwise (msa_nw_set_wait).
+constexpr uint32_t kStripWaitUs = 5000000;
 // Entries of a boundary row's base table for ncols columns, and the tables it
 // has: strip s writes table s mod 8 and reads the one before. A chained strip is
 // at least 128 steps behind the one it follows when it moves its base, so the
@@ -400,6 +401,7 @@ struct BatchParams {
     const uint64_t *chain_off;
     uint32_t *chain_flag;
     int *err;                   // set when a wait between strips ran out
+    unsigned long long wait_ns; // limit of those waits
     uint32_t step;              // largest s + 2g, for the moving base
 };
 
@@ -748,12 +750,13 @@ struct Chain {
     const uint32_t *above;
     uint32_t *mine;
     int *err;
+    unsigned long long wait_ns;
 };
 
 // Waits until *flag >= want and returns its value, or gives up: then, and in
 // every later wait of the launch, the strip runs on with what is there and the
 // call fails.
-__device__ __noinline__ uint32_t chain_wait(const uint32_t *flag, uint32_t want, int *err)
+__device__ __noinline__ uint32_t chain_wait(const uint32_t *flag, uint32_t want, int *err, unsigned long long wait_ns)
 {
     unsigned long long t0, t1;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
@@ -762,7 +765,7 @@ __device__ __noinline__ uint32_t chain_wait(const uint32_t *flag, uint32_t want,
         if(v >= want) return v;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
         if(*(volatile int *) err != 0) return want;
-        if(t1 - t0 > kChainWaitNs) {
+        if(t1 - t0 > wait_ns) {
             atomicExch(err, 1);
             return want;
         }
@@ -804,7 +807,7 @@ __device__ __forceinline__ void sweep_long(const uint32_t *__restrict__ sprof, c
         if(first) return 0u;
         if(chain.above) {
             const uint32_t want = (uint32_t) min(c0 + 32, ncols);
-            if(known < want) known = chain_wait(chain.above, want, chain.err);
+            if(known < want) known = chain_wait(chain.above, want, chain.err, chain.wait_ns);
         }
         const int c = c0 + lane;
         if(c >= ncols) return 0u;
@@ -1148,7 +1151,7 @@ template <int RMAX, int W, bool kPack>
 __device__ __forceinline__ void rows_pair_task(const JobView &jv, uint32_t k, uint32_t grp, uint32_t ngrp,
                                                uint32_t *sprof_b, uint32_t *bound, int warp, int lane,
                                                uint64_t words = 0, uint32_t step = 0, int strip = -1,
-                                               const dev::Chain &chain = dev::Chain{nullptr, nullptr, nullptr})
+                                               const dev::Chain &chain = dev::Chain{nullptr, nullptr, nullptr, 0})
 {
     const uint32_t a1 = 2 * k, a2 = min(2 * k + 1, jv.nclean - 1);
     const uint32_t x1 = jv.sorted[a1], x2 = jv.sorted[a2];
@@ -1260,7 +1263,7 @@ __global__ void __launch_bounds__(W * 32, BatchOcc<RMAX, W>::value) nw_batched_k
                 const uint32_t grp = qq / nst, strip = qq - grp * nst;
                 const uint64_t words = chain_words_of(second);
                 uint32_t *flag = p.chain_flag + task_q * W + warp;
-                const dev::Chain chain{strip ? flag - W : nullptr, flag, p.err};
+                const dev::Chain chain{strip ? flag - W : nullptr, flag, p.err, p.wait_ns};
                 rows_pair_task<RMAX, W, kPack>(p.job, lo, grp, 1, sprof_b,
                                                p.chain_bound + p.chain_off[lo] + (grp * W + warp) * words, warp, lane,
                                                words, p.step, (int) strip, chain);
@@ -1540,6 +1543,7 @@ struct NwPlan {
     uint32_t part = 0, nparts = 1;
     int variant = 0;            // msa_nw_set_variant flags the plan was built with
     uint32_t chunk = 0;         // and its groups-per-task override
+    uint32_t wait_us = 0;       // and its waits (msa_nw_set_wait)
     size_t clear_bytes = 64;    // of the work counter and what follows it
     bool chained = false;
     bool profiles = true;       // whether any kernel of the plan reads score profiles
@@ -1649,6 +1653,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     pl->nparts = nparts;
     pl->variant = ctx->nw_variant;
     pl->chunk = ctx->nw_chunk;
+    pl->wait_us = ctx->nw_wait_us;
 
     const uint32_t nclean = (uint32_t) st->clean_sorted.size();
     const uint64_t nclean_pairs = (uint64_t) nclean * (nclean > 0 ? nclean - 1 : 0) / 2;
@@ -1918,6 +1923,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     bp.bound_stride = stride;
     bp.counter = (unsigned long long *) (base + o_cnt);
     bp.err = (int *) (base + o_cnt + 8);
+    bp.wait_ns = (unsigned long long) (ctx->nw_wait_us ? ctx->nw_wait_us : kStripWaitUs) * 1000ull;
     bp.chain_flag = (uint32_t *) (base + o_cnt + 64);
     bp.chain_bound = (uint32_t *) (base + o_cb);
     bp.chain_off = (const uint64_t *) (base + o_co);
@@ -1948,6 +1954,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
         q.g = tbl.penalty;
         q.nchain = (uint32_t) bits.nchain;
         q.err = bp.err;
+        q.wait_ns = bp.wait_ns;
         q.counter = (unsigned long long *) (base + o_cnt + 16);   // cleared with the batched kernel's
     }
 
@@ -2046,7 +2053,7 @@ int nw_run(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode, int32_t *d
         NwPlan *c = plans[i];
         if(c->store_serial == st->serial && c->mode == mode && c->d_out == d_out && c->tiles.R == tiles.R &&
            c->tiles.W == tiles.W && c->part == part && c->nparts == nparts && same_table(c->tbl, tbl) &&
-           c->variant == ctx->nw_variant && c->chunk == ctx->nw_chunk) {
+           c->variant == ctx->nw_variant && c->chunk == ctx->nw_chunk && c->wait_us == ctx->nw_wait_us) {
             pl = c;
             plans.erase(plans.begin() + i);
             plans.push_back(pl);

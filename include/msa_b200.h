@@ -189,6 +189,12 @@ int msa_nw_all_pairs_part(msa_ctx *ctx, msa_seqs seqs, const msa_table *table, i
 int msa_nw_part_of_pairs(const uint8_t *units, const uint64_t *offs, const uint64_t *lens, uint32_t n,
                          const msa_table *table, uint32_t nparts, uint32_t *out_part);
 
+/* Gives back the device memory that the context keeps for later calls: plans of
+ * earlier calls (at most 2 GiB beyond the newest) and free blocks (at most
+ * 1 GiB). Allocations of the context that fail do this by themselves. No
+ * counterpart in the reference. */
+int msa_release_idle(msa_ctx *ctx);
+
 /* Tile shape of the persistent kernel: rows per lane (16 or 32) and warps per
  * CTA (4 or 8); 0, 0 restores the committed autotuned choice. No counterpart
  * in the reference (its one kernel shape is fixed, hybrid.cu:57). */

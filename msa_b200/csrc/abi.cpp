@@ -12,12 +12,17 @@
 
 namespace msa {
 
-cudaError_t DevBuf::ensure(size_t need)
+cudaError_t DevBuf::ensure(size_t need, msa_ctx *keeper)
 {
     if(need <= bytes && ptr) return cudaSuccess;
     if(ptr) { cudaFree(ptr); ptr = nullptr; bytes = 0; }
     size_t want = std::max<size_t>(need, 256);
     cudaError_t e = cudaMalloc(&ptr, want);
+    if(e != cudaSuccess && keeper) {
+        cudaGetLastError();
+        release_idle(keeper);
+        e = cudaMalloc(&ptr, want);
+    }
     if(e != cudaSuccess) { ptr = nullptr; bytes = 0; cudaGetLastError(); return e; }
     bytes = want;
     return cudaSuccess;
@@ -43,12 +48,7 @@ cudaError_t BlockCache::take(size_t need, void **ptr, size_t *bytes)
             m_free.erase(m_free.begin() + k);
             return cudaSuccess;
         }
-    cudaError_t e = cudaMalloc(ptr, want);
-    if(e != cudaSuccess && !m_free.empty()) {
-        cudaGetLastError();
-        clear();
-        e = cudaMalloc(ptr, want);
-    }
+    const cudaError_t e = cudaMalloc(ptr, want);
     if(e != cudaSuccess) {
         cudaGetLastError();
         *ptr = nullptr;
@@ -84,6 +84,22 @@ void BlockCache::clear()
     for(const Block &b : m_free) cudaFree(b.ptr);
     m_free.clear();
     m_total = 0;
+}
+
+cudaError_t take_block(msa_ctx *ctx, size_t need, void **ptr, size_t *bytes)
+{
+    cudaError_t e = ctx->blocks.take(need, ptr, bytes);
+    if(e != cudaSuccess) {
+        release_idle(ctx);
+        e = ctx->blocks.take(need, ptr, bytes);
+    }
+    return e;
+}
+
+void release_idle(msa_ctx *ctx)
+{
+    drop_plans(ctx);
+    ctx->blocks.clear();
 }
 
 int set_error(msa_ctx *ctx, int status, const std::string &msg)
@@ -166,6 +182,15 @@ void msa_destroy(msa_ctx *ctx)
     for(auto &e : ctx->ev) if(e) cudaEventDestroy(e);
     if(ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
+}
+
+int msa_release_idle(msa_ctx *ctx)
+{
+    if(!ctx) return MSA_ERR_INVALID;
+    cudaSetDevice(ctx->device);
+    cudaStreamSynchronize(ctx->stream);
+    release_idle(ctx);
+    return MSA_OK;
 }
 
 const char *msa_last_error(const msa_ctx *ctx) { return ctx ? ctx->err.c_str() : ""; }
@@ -258,7 +283,7 @@ int build_store(msa_ctx *ctx, const uint8_t *units, const uint64_t *offs, const 
         st->home = ctx;
         cudaStream_t s = ctx->stream;
         cudaError_t e = st->pooled ? cudaMallocFromPoolAsync(&st->block, at, ctx->pool, s)
-                                   : ctx->blocks.take(at, &st->block, &st->block_bytes);
+                                   : take_block(ctx, at, &st->block, &st->block_bytes);
         if(e) st->block = nullptr;
         if(!e) {
             uint8_t *base = (uint8_t *) st->block;
@@ -406,7 +431,7 @@ static int all_pairs(msa_ctx *ctx, msa_seqs seqs, const msa_table *table, int mo
         } reorient(st, !table_is_symmetric(ext));
         int32_t *d_out = out;
         if(!out_on_device && npairs) {
-            cudaError_t e = ctx->out_tmp.ensure(npairs * sizeof(int32_t));
+            cudaError_t e = ctx->out_tmp.ensure(npairs * sizeof(int32_t), ctx);
             if(e) return cuda_error(ctx, e, "output buffer");
             d_out = (int32_t *) ctx->out_tmp.ptr;
         }

@@ -58,6 +58,19 @@ msa_ctx *context_for(int dev)
 
 thread_local int t_device = 0;
 
+// Device memory of the selected device, after its context has given back what it keeps
+// where there is none left.
+cudaError_t device_malloc(void **ptr, size_t bytes, int dev)
+{
+    cudaError_t e = cudaMalloc(ptr, bytes);
+    if(e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        msa_release_idle(context_for(dev));
+        e = cudaMalloc(ptr, bytes);
+    }
+    return e;
+}
+
 __global__ void accumulate_kernel(int32_t *out, const int32_t *part, uint64_t n)
 {
     for(uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t) gridDim.x * blockDim.x)
@@ -387,7 +400,7 @@ distance_matrix score(const database &db, const scoring_table &table, int mode, 
     auto st = std::make_shared<distance_matrix::storage>();
     st->device = home;
     check_cuda(cudaSetDevice(home), "select device");
-    check_cuda(cudaMalloc((void **) &st->dev, std::max<uint64_t>(np * 4, 16)), "allocate distance matrix");
+    check_cuda(device_malloc((void **) &st->dev, std::max<uint64_t>(np * 4, 16), home), "allocate distance matrix");
     const int ndev = device::count();
     devices = std::max(1, std::min(devices, ndev));
 
@@ -416,7 +429,7 @@ distance_matrix score(const database &db, const scoring_table &table, int mode, 
         workers.emplace_back([&, k, dev] {
             try {
                 check_cuda(cudaSetDevice(dev), "select device");
-                check_cuda(cudaMalloc((void **) &bufs[k], np * 4), "allocate part");
+                check_cuda(device_malloc((void **) &bufs[k], np * 4, dev), "allocate part");
                 check_cuda(cudaMemset(bufs[k], 0, np * 4), "clear part");
                 run_part(dev, (uint32_t) k, bufs[k]);
             } catch(const std::exception &e) {
@@ -430,7 +443,7 @@ distance_matrix score(const database &db, const scoring_table &table, int mode, 
     int32_t *staging = nullptr;
     if(err.empty()) {
         check_cuda(cudaSetDevice(home), "select device");
-        check_cuda(cudaMalloc((void **) &staging, np * 4), "allocate staging");
+        check_cuda(device_malloc((void **) &staging, np * 4, home), "allocate staging");
         for(int k = 0; k < devices && err.empty(); ++k) {
             const int dev = (home + k) % ndev;
             const cudaError_t e = cudaMemcpyPeer(staging, home, bufs[k], dev, np * 4);
@@ -486,7 +499,7 @@ distance_matrix run(const device_database &db, const scoring_table &table, const
     auto st = std::make_shared<distance_matrix::storage>();
     st->device = db.device();
     check_cuda(cudaSetDevice(db.device()), "select device");
-    check_cuda(cudaMalloc((void **) &st->dev, std::max<uint64_t>(np * 4, 16)), "allocate distance matrix");
+    check_cuda(device_malloc((void **) &st->dev, std::max<uint64_t>(np * 4, 16), db.device()), "allocate distance matrix");
     msa_ctx *c = context_for(db.device());
     check_status(msa_nw_all_pairs(c, db.handle(), &table.raw(), mode, st->dev, 1), c);
     return make_device_matrix(st, n);

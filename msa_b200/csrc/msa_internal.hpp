@@ -89,7 +89,8 @@ struct SeqStore {
 struct DevBuf {
     void *ptr = nullptr;
     size_t bytes = 0;
-    cudaError_t ensure(size_t need);
+    // `keeper`: the context whose idle memory is given back when there is none left.
+    cudaError_t ensure(size_t need, msa_ctx *keeper = nullptr);
     void release();
 };
 
@@ -98,7 +99,7 @@ struct DevBuf {
 // small call. Sizes are rounded up to quarters of a power of two so that
 // similar calls share them. Used by the context's thread only, and only for
 // blocks that no work in flight touches. Holds at most kCacheBytes in
-// kCacheBlocks blocks; emptied when an allocation fails and with the context.
+// kCacheBlocks blocks; emptied by release_idle and with the context.
 class BlockCache {
 public:
     cudaError_t take(size_t need, void **ptr, size_t *bytes);
@@ -195,6 +196,13 @@ constexpr int kUnitFront = 64;
 int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order, msa_otu *out);
 
 void release_graphs(msa_ctx *ctx);
+// Drops every kept plan (of calls that are over).
+void drop_plans(msa_ctx *ctx);
+// Gives back the device memory that a context keeps for later calls: plans and free
+// blocks. Allocations of its own that fail do this and are tried once more.
+void release_idle(msa_ctx *ctx);
+// A block of the context's cache (BlockCache::take).
+cudaError_t take_block(msa_ctx *ctx, size_t need, void **ptr, size_t *bytes);
 int build_store(msa_ctx *ctx, const uint8_t *units, const uint64_t *offs, const uint64_t *lens, uint32_t n,
                 SeqStore **out);
 void destroy_store(SeqStore *st);

@@ -928,7 +928,7 @@ static int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order
                  // flags between clusters: pub_seq, pub_xy[2], cand_seq[], cand[][][2]
                  oSync = take(helped ? 64 + (size_t) kMaxHelperCtas * 4 : 0),
                  oCand = take(helped ? (size_t) 2 * kMaxHelperCtas * 16 : 0);
-    MSA_CUDA_TRY(ctx, ctx->nj_buf.ensure(off));
+    MSA_CUDA_TRY(ctx, ctx->nj_buf.ensure(off, ctx));
     char *base = (char *) ctx->nj_buf.ptr;
     // Head: phase counters, the error word, the largest |D|.
     unsigned long long *d_cycles = (unsigned long long *) (base + oHead);
@@ -1056,7 +1056,7 @@ static int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order
         K = pick_cluster(kern_help, kThreads, [&](unsigned) { return (size_t) pitch(m) * 16; }, &resident);
         void *D = nullptr;
         size_t bytes = 0;
-        if(K < 2 || ctx->blocks.take((size_t) (m + 1) * pitch(m) * 4, &D, &bytes))
+        if(K < 2 || take_block(ctx, (size_t) (m + 1) * pitch(m) * 4, &D, &bytes))
             return nj_run(ctx, tri, kind, n, order, false, out);
         cudaError_t e = cudaMemsetAsync(d_err, 0, 4, s);
         compact_kernel<<<std::min<uint32_t>(m + 1, 4 * (uint32_t) ctx->num_sms), 256, 0, s>>>(

@@ -1606,6 +1606,13 @@ void release_graphs(msa_ctx *ctx)
     ctx->graphs = nullptr;
 }
 
+void drop_plans(msa_ctx *ctx)
+{
+    if(!ctx->graphs) return;
+    for(NwPlan *pl : ctx->graphs->plans) ctx->graphs->drop(pl);
+    ctx->graphs->plans.clear();
+}
+
 void drop_plans_for_store(msa_ctx *ctx, uint64_t serial)
 {
     if(!ctx->graphs) return;
@@ -1867,7 +1874,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
                  o_bb = take(pl->bits_grid * kBitWarps * bits.bound_words * sizeof(uint2)),
                  // the work counter, the error word and the chained strips' progress, cleared by every launch
                  o_cnt = take(64 + chain_tasks * 8 * sizeof(uint32_t));
-    MSA_CUDA_TRY(ctx, ctx->blocks.take(off, &pl->mem, &pl->mem_bytes));
+    MSA_CUDA_TRY(ctx, take_block(ctx, off, &pl->mem, &pl->mem_bytes));
     pl->home = ctx;
     char *base = (char *) pl->mem;
     cudaStream_t s = ctx->stream;

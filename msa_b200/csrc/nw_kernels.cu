@@ -1744,7 +1744,8 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
         auto eff_at = [&](uint32_t a) { return (uint64_t) st->eff[st->clean_sorted[std::min(a, nrows - 1)]]; };
         // Rows of rows pair k, and its longest column sequence.
         auto rows_at = [&](uint32_t k) { return std::max(eff_at(2 * k), eff_at(2 * k + 1)); };
-        auto cols_at = [&](uint32_t k) { return gap || !table_is_symmetric(tbl) ? (eff_at(2 * k + 1) + 2) / 3 * 3 : eff_at(2 * k + 1); };
+        const bool oriented = gap || !table_is_symmetric(tbl);
+        auto cols_at = [&](uint32_t k) { return oriented ? (eff_at(2 * k + 1) + 2) / 3 * 3 : eff_at(2 * k + 1); };
         row_narrow.assign(K, 0);
         std::vector<uint64_t> groups_k(K, 0);
         for(uint32_t k = 0; k < K; ++k) {

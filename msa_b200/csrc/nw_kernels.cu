@@ -356,10 +356,9 @@ struct JobView {
 // row_narrow flags: 16-bit lanes; rows pairs k and k + 1 (kRowQuad), or k to
 // k + 3 (kRowOct), stacked in one warp (stack_task), their tasks all under k.
 // Rows pairs of several strips: kRowLong runs its 16-bit lanes on a moving base
-// (sweep_long), kRowChain makes every strip a task of its own, of 32 x 32, 16 or
-// 8 rows (chain_rows).
-constexpr uint8_t kRowNarrow = 1, kRowQuad = 2, kRowLong = 4, kRowChain = 8, kRowR16 = 16, kRowR8 = 32,
-                  kRowOct = 64;
+// (sweep_long), kRowChain makes every strip a task of its own, of up to 32 x 32
+// rows or 32 x 16 (chain_form).
+constexpr uint8_t kRowNarrow = 1, kRowQuad = 2, kRowLong = 4, kRowChain = 8, kRowR16 = 16, kRowOct = 64;
 
 // Steps between moves of a long strip's base; see sweep_long.
 constexpr int kRebase = 512;
@@ -1124,12 +1123,11 @@ __device__ __forceinline__ void strip_plan(int rows, int &nst, int &R)
 }  // namespace dev
 
 // Rows per lane of a rows pair's strips, from its flags: the plan's, or for a
-// chained one that would leave SMs idle, 16 or 8.
+// chained one with lower strips, 16.
 template <int RMAX>
 __host__ __device__ __forceinline__ int strip_rows(int rows, uint8_t flags)
 {
     if(flags & kRowR16) return 16;
-    if(flags & kRowR8) return 8;
     const int nst = (rows + 32 * RMAX - 1) / (32 * RMAX);
     const int R = (rows + 32 * nst - 1) / (32 * nst);
     return (R + 1) & ~1;
@@ -1197,8 +1195,8 @@ __device__ __forceinline__ void rows_pair_task(const JobView &jv, uint32_t k, ui
             const int8_t *g1 = jv.prof + jv.poff[x1], *g2 = jv.prof + jv.poff[x2];
             const uint32_t lp1 = jv.plp[x1], lp2 = jv.plp[x2];
 #define MSA_LONG(RR) case RR: dev::long_task<RR, kPack>(sprof_b, g1, lp1, g2, lp2, e1, e2, s0, s1, tc, bound, words, chain, step, jv.g, lane); break;
-            switch(R) {   // strips of several per rows pair: 18 rows per lane and more, or 16 or 8
-                MSA_LONG(8) MSA_LONG(16) MSA_LONG(18) MSA_LONG(20) MSA_LONG(22) MSA_LONG(24) MSA_LONG(26) MSA_LONG(28)
+            switch(R) {   // strips of several per rows pair: 18 rows per lane and more, or 16
+                MSA_LONG(16) MSA_LONG(18) MSA_LONG(20) MSA_LONG(22) MSA_LONG(24) MSA_LONG(26) MSA_LONG(28)
                 MSA_LONG(30) MSA_LONG(32) default: break;
             }
 #undef MSA_LONG
@@ -1649,6 +1647,41 @@ static void launch_batched(const NwPlan &pl, cudaStream_t s)
     nw_batched_kernel<R, W, kPack><<<(unsigned) pl.batch_grid, W * 32, smem, s>>>(pl.bp);
 }
 
+// Whether the longest rows pairs are chained, and with strips of how many rows: the
+// form with the least estimated time, from the longest of them (`rows`, `columns`;
+// `moving`: on a moving base also when not chained), the column groups of all of them,
+// their strips of up to 1,024 rows and of 512, and the resident CTAs. In units of a
+// step's instructions: a strip is columns + 31 steps of (rows per lane + 28), 28 more
+// on a moving base; a strip follows the one above by about 70 steps more than its own
+// lanes need. Up to one CTA per SM run undisturbed; two share the SM's shared-memory
+// pipe; beyond that tasks wait for a CTA, and chained ones that wait for each other
+// hold theirs. The factors are fitted to 104 jobs of 2 to 700 sequences of up to 60,000
+// residues, each measured unchained, with strips of 1,024 and of 512 rows: the form
+// taken is within 1% of the best in the mean and 23% at worst. Chaining wherever the
+// launch's share allows, with strips as low as 256 rows where the CTAs are not all
+// taken, was 15% slower in the mean: 64 sequences of 1,030 residues 528 us (299 not
+// chained), one of 20,000 among 49 of 200 2.37 ms (0.94 not chained, 0.71 with strips
+// of 1,024 rows), 24 of 6,000 2.57 ms (6.95, 1.46).
+static uint8_t chain_form(uint64_t rows, uint64_t columns, bool moving, uint64_t groups, uint64_t strips, uint64_t low,
+                          uint64_t resident)
+{
+    const double steps = (double) columns + 31, full = (double) resident;
+    auto strip = [&](int R, bool base) { return steps * (R + 28 + (base ? 28 : 0)); };
+    auto share = [&](uint64_t n, double two, double slope) {
+        return 2 * n <= resident ? 1.0 : n <= resident ? two : 0.5 + slope * (double) n / full;
+    };
+    auto chained = [&](uint64_t nst, int R, uint64_t tasks) {
+        const double line = (double) ((tasks + resident - 1) / resident) * (1.0 + (double) (nst - 1) * 70.0 / steps);
+        return std::max(share(tasks, 1.35, 1.25), line) * strip(R, true);
+    };
+    const int R = strip_rows<32>((int) rows, 0);
+    const uint64_t nst = (rows + 32 * R - 1) / (32 * (uint64_t) R);
+    const double apart = (double) nst * strip(R, moving) * share(groups, 1.65, 1.8);
+    const double high = chained(nst, R, strips), halved = chained((rows + 511) / 512, 16, low);
+    if(apart <= std::min(high, halved)) return 0;
+    return high <= halved ? kRowLong | kRowChain : kRowLong | kRowChain | kRowR16;
+}
+
 static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode, int32_t *d_out, Tiles tiles,
                       uint32_t part, uint32_t nparts, NwPlan *pl)
 {
@@ -1790,12 +1823,11 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
         }
         // Where the strips of the longest rows pair, one after the other, take
         // more than the launch's share per resident CTA, it and those down to
-        // half of that share are chained: every strip a task, each waiting for
+        // half of that share may be chained: every strip a task, each waiting for
         // the boundary row of the one above as it comes. (50 genomes: 4.7 ms,
         // 5.4 when only those above the whole share are; where the longest is
         // below it, the order of the tasks balances them, and chaining would
-        // cost 1,200 uneven sequences 0.3%.) Where the strips are too few for
-        // the CTAs, they are made lower.
+        // cost 1,200 uneven sequences 0.3%.)
         chain_off.assign(K + 1, 0);
         const uint64_t resident = 2 * (uint64_t) ctx->num_sms;
         if(tiles.R == 32 && tiles.W == 8 && !ctx->nw_variant && !ctx->tile_r && long_ok(tbl, gap)) {
@@ -1807,18 +1839,26 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
             uint64_t total = 0;
             for(uint32_t k = k_lo; k < k_hi; ++k) total += groups_k[k] * task_cost(k);
             uint32_t kc = k_lo;
-            uint64_t strips = 0;
+            uint64_t groups = 0, strips = 0, low = 0;
             for(; kc < k_hi; ++kc) {
                 const uint64_t rows = rows_at(kc), words = groups_k[kc] * 8 * chain_words_of((uint32_t) eff_at(2 * kc + 1));
                 if(rows <= 32 * 32 || !row_narrow[kc] || (kc == k_lo ? 1 : 2) * resident * task_cost(kc) < total) break;
                 if(chain_words + words > (kChainBytes >> 2)) break;
                 chain_off[kc] = chain_words;
                 chain_words += words;
+                groups += groups_k[kc];
                 strips += groups_k[kc] * ((rows + 1023) / 1024);
+                low += groups_k[kc] * ((rows + 511) / 512);
             }
-            const uint8_t lower = strips >= resident ? 0 : 2 * strips >= resident ? kRowR16 : kRowR8;
+            const uint8_t form = kc == k_lo ? 0 : chain_form(rows_at(k_lo), cols_at(k_lo), row_narrow[k_lo] & kRowLong, groups,
+                                                             strips, low, resident);
+            if(!(form & kRowChain)) {
+                kc = k_lo;
+                chain_words = 0;
+                chain_off.assign(K + 1, 0);
+            }
             for(uint32_t k = k_lo; k < kc; ++k) {
-                row_narrow[k] |= kRowLong | kRowChain | lower;
+                row_narrow[k] |= form;
                 const uint64_t SH = 32 * (uint64_t) strip_rows<32>((int) rows_at(k), row_narrow[k]);
                 groups_k[k] *= (rows_at(k) + SH - 1) / SH;   // tasks
                 chain_tasks += groups_k[k];

@@ -78,26 +78,17 @@ __device__ __forceinline__ int count_bits(uint32_t x, int lane)
     return __popc(x);
 }
 
-// Progress of the warps of a CTA that share a task's strips, as strip_progress gives
-// it (null: one warp has all of them).
-struct Strips {
-    volatile unsigned long long *done;
-    int *err;
-    unsigned long long wait_ns;   // limit of a strip's wait for the one above it
-};
-
 // Waits until *done >= want, or gives up: then, and in every later wait of the
 // launch, the strip runs on with what is there and the call fails.
-__device__ __noinline__ void strip_wait(volatile unsigned long long *done, unsigned long long want, int *err,
-                                        unsigned long long wait_ns)
+__device__ __noinline__ void strip_wait(const BitParams &p, volatile unsigned long long *done, unsigned long long want)
 {
     unsigned long long t0, t1;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
     while(*done < want) {
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-        if(*(volatile int *) err != 0) break;
-        if(t1 - t0 > wait_ns) {
-            atomicExch(err, 1);
+        if(*(volatile int *) p.err != 0) break;
+        if(t1 - t0 > p.wait_ns) {
+            atomicExch(p.err, 1);
             break;
         }
         __nanosleep(100);
@@ -106,11 +97,13 @@ __device__ __noinline__ void strip_wait(volatile unsigned long long *done, unsig
 
 // One task. `ring`: the warp's kRingRows rows of S words. S is 0 mod 32 where the
 // lanes are on 32 different columns, and 8 or 16 where 4 or 2 lanes are on one: equal
-// columns of the first letters then lie in different banks.
+// columns of the first letters then lie in different banks. `done`: the progress of the
+// warps of a CTA that share a task's strips, as strip_progress gives it (null: one warp
+// has all of them).
 template <int R, int LP>
 __device__ __noinline__ void bit_task(const BitParams &p, const BitSet &set, uint32_t grp, uint32_t *ring,
                                       uint2 *bound, int lane, int s0 = 0, int ds = 1,
-                                      const Strips &strips = Strips{nullptr, nullptr, 0})
+                                      volatile unsigned long long *done = nullptr)
 {
     constexpr int S = 96 + (LP == 8 ? 8 : LP == 16 ? 16 : 0), U = R <= 8 ? 4 : R <= 16 ? 2 : 1;
     const int at = lane % LP, ncols = (int) p.gcols[grp];
@@ -167,16 +160,16 @@ __device__ __noinline__ void bit_task(const BitParams &p, const BitSet &set, uin
                     dst[32] = w[q];
                 }
             }
-            if(LP == 32 && strips.done) {
+            if(LP == 32 && done) {
                 // Lane 31 has stored the columns up to c0 - 32.
                 if(lane == 31 && c0 > 31) {
                     __threadfence_block();
-                    strips.done[st % ds] = strip_progress((uint32_t) st, (uint32_t) (c0 - 31));
+                    done[st % ds] = strip_progress((uint32_t) st, (uint32_t) (c0 - 31));
                 }
                 if(st > 0) {
                     const unsigned long long want = strip_progress((uint32_t) st - 1, (uint32_t) min(c0 + 32, ncols));
-                    if(strips.done[(st - 1) % ds] < want)
-                        strip_wait(strips.done + (st - 1) % ds, want, strips.err, strips.wait_ns);
+                    if(done[(st - 1) % ds] < want)
+                        strip_wait(p, done + (st - 1) % ds, want);
                     __threadfence_block();
                 }
                 __syncwarp();
@@ -221,9 +214,9 @@ __device__ __noinline__ void bit_task(const BitParams &p, const BitSet &set, uin
             }
         }
         __syncwarp();
-        if(LP == 32 && strips.done && lane == 31) {
+        if(LP == 32 && done && lane == 31) {
             __threadfence_block();
-            strips.done[st % ds] = strip_progress((uint32_t) st, 0xffffffffu);
+            done[st % ds] = strip_progress((uint32_t) st, 0xffffffffu);
         }
     }
     if((nst - 1) % ds != s0) return;   // another warp has the last row
@@ -332,8 +325,7 @@ __global__ void __launch_bounds__(kBitWarps * 32, 4) nw_bits_kernel(BitParams p)
         const BitSet set = find((uint32_t) q);
         const uint32_t grp = max(p.g0, set.a / 32) + (uint32_t) q - set.first;
         uint2 *bound = p.bound + blockIdx.x * kBitWarps * p.bound_words;
-        const dev::Strips strips{done, p.err, p.wait_ns};
-#define MSA_BITS(RR) case RR: dev::bit_task<RR, 32>(p, set, grp, ring, bound, lane, warp, kBitWarps, strips); break;
+#define MSA_BITS(RR) case RR: dev::bit_task<RR, 32>(p, set, grp, ring, bound, lane, warp, kBitWarps, done); break;
         if(warp < (int) set.nst)
             switch(set.R) {
                 MSA_BITS(18) MSA_BITS(20) MSA_BITS(22) MSA_BITS(24) MSA_BITS(26) MSA_BITS(28) MSA_BITS(30) MSA_BITS(32)

@@ -795,6 +795,15 @@ __global__ void __launch_bounds__(kThreads, 1) nj_cluster_kernel(State st)
     cluster.sync();   // no CTA leaves while another may still write its shared memory
 }
 
+// Lets a kernel be launched with up to kMaxSmem bytes of dynamic shared memory. The
+// same value on every call: the attribute belongs to the process, and threads with
+// contexts of their own launch the same kernels with different sizes.
+template <class Kern>
+cudaError_t allow_smem(Kern kern)
+{
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kMaxSmem);
+}
+
 // Largest cluster (16, 8, 4 or 2 CTAs) of `kern` that can be resident with
 // smem(k) bytes of dynamic shared memory per CTA, and how many of them; 0 if none.
 template <class Kern, class Smem>
@@ -803,7 +812,7 @@ unsigned pick_cluster(Kern kern, unsigned threads, Smem smem, int *clusters)
     for(unsigned k : {16u, 8u, 4u, 2u}) {
         const size_t bytes = smem(k);
         if(bytes > kMaxSmem) continue;
-        if(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes) != cudaSuccess ||
+        if(allow_smem(kern) != cudaSuccess ||
            cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
             cudaGetLastError();
             continue;
@@ -1031,7 +1040,7 @@ static int nj_run(msa_ctx *ctx, const void *tri, int kind, uint32_t n, int order
                 const int threads = st.N <= kTinyNodes ? 128 : 512;
                 auto kern_small = st.N <= kTinyNodes ? (linear ? nj_small_kernel<true, 128> : nj_small_kernel<false, 128>)
                                                      : (linear ? nj_small_kernel<true, 512> : nj_small_kernel<false, 512>);
-                MSA_CUDA_TRY(ctx, cudaFuncSetAttribute(kern_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes));
+                MSA_CUDA_TRY(ctx, allow_smem(kern_small));
                 kern_small<<<1, threads, bytes, s>>>(st);
                 MSA_CUDA_TRY(ctx, cudaGetLastError());
                 ctx->launches++;

@@ -1647,39 +1647,43 @@ static void launch_batched(const NwPlan &pl, cudaStream_t s)
     nw_batched_kernel<R, W, kPack><<<(unsigned) pl.batch_grid, W * 32, smem, s>>>(pl.bp);
 }
 
+// Instructions of a warp's step besides its cells, and what a moving base adds.
+constexpr uint64_t kStepCost = 28, kMovingCost = 22;
+
 // Whether the longest rows pairs are chained, and with strips of how many rows: the
 // form with the least estimated time, from the longest of them (`rows`, `columns`;
-// `moving`: on a moving base also when not chained), the column groups of all of them,
-// their strips of up to 1,024 rows and of 512, and the resident CTAs. In units of a
-// step's instructions: a strip is columns + 31 steps of (rows per lane + 28), 28 more
-// on a moving base; a strip follows the one above by about 70 steps more than its own
-// lanes need. Up to one CTA per SM run undisturbed; two share the SM's shared-memory
-// pipe; beyond that tasks wait for a CTA, and chained ones that wait for each other
-// hold theirs. The factors are fitted to 104 jobs of 2 to 700 sequences of up to 60,000
-// residues, each measured unchained, with strips of 1,024 and of 512 rows: the form
-// taken is within 1% of the best in the mean and 23% at worst. Chaining wherever the
-// launch's share allows, with strips as low as 256 rows where the CTAs are not all
-// taken, was 15% slower in the mean: 64 sequences of 1,030 residues 528 us (299 not
-// chained), one of 20,000 among 49 of 200 2.37 ms (0.94 not chained, 0.71 with strips
-// of 1,024 rows), 24 of 6,000 2.57 ms (6.95, 1.46).
-static uint8_t chain_form(uint64_t rows, uint64_t columns, bool moving, uint64_t groups, uint64_t strips, uint64_t low,
-                          uint64_t resident)
+// `moving`: on a moving base also when not chained) and the work of all rows pairs as
+// one task each (`tasks`), of the chained ones' strips of up to 1,024 rows (`high`) and
+// of 512 (`low`), counted in the longest's own tasks or strips. A strip is columns + 31
+// steps; it follows the one above by about 100 steps more than its own lanes need. Up to
+// one CTA per SM runs undisturbed, two share the SM's shared-memory pipe, and beyond
+// that tasks wait for a CTA; strips that wait for each other hold theirs. The factors
+// are fitted to 178 jobs of 2 to 700 sequences of up to 60,000 residues, alike, log-normal
+// and one long among short ones, each measured unchained, with strips of 1,024 and of
+// 512 rows: the form taken is within 2.1% of the best in the mean and 24% at worst, and
+// nowhere more than 9% slower than unchained. Chaining wherever the launch's share
+// allows, with strips as low as 256 rows where they do not fill the CTAs, was 12% slower
+// in the mean: 64 sequences of 1,030 residues 528 us (299 not chained), one of 20,000
+// among 49 of 200 2.37 ms (0.94 not chained, 0.71 with strips of 1,024 rows), 24 of 6,000
+// 2.57 ms (6.95, 1.46).
+static uint8_t chain_form(uint64_t rows, uint64_t columns, bool moving, double tasks, double high, double low,
+                          double resident)
 {
-    const double steps = (double) columns + 31, full = (double) resident;
-    auto strip = [&](int R, bool base) { return steps * (R + 28 + (base ? 28 : 0)); };
-    auto share = [&](uint64_t n, double two, double slope) {
-        return 2 * n <= resident ? 1.0 : n <= resident ? two : 0.5 + slope * (double) n / full;
+    const double steps = (double) columns + 31;
+    auto share = [&](double n, double two, double base, double slope) {
+        return 2 * n <= resident ? 1.0 : n <= resident ? two : std::max(two, base + slope * n / resident);
     };
-    auto chained = [&](uint64_t nst, int R, uint64_t tasks) {
-        const double line = (double) ((tasks + resident - 1) / resident) * (1.0 + (double) (nst - 1) * 70.0 / steps);
-        return std::max(share(tasks, 1.35, 1.25), line) * strip(R, true);
+    auto chained = [&](uint64_t nst, int R, double n) {
+        const double line = std::max(1.0, n / resident) * (1.0 + (double) (nst - 1) * 100.0 / steps);
+        return std::max(share(n, 1.25, 0.3, 1.5), line) * steps * (double) (R + kStepCost + kMovingCost);
     };
     const int R = strip_rows<32>((int) rows, 0);
     const uint64_t nst = (rows + 32 * R - 1) / (32 * (uint64_t) R);
-    const double apart = (double) nst * strip(R, moving) * share(groups, 1.65, 1.8);
-    const double high = chained(nst, R, strips), halved = chained((rows + 511) / 512, 16, low);
-    if(apart <= std::min(high, halved)) return 0;
-    return high <= halved ? kRowLong | kRowChain : kRowLong | kRowChain | kRowR16;
+    const double apart = (double) nst * steps * (double) (R + kStepCost + (moving ? kMovingCost : 0)) *
+                         share(tasks, 1.65, 0.5, 1.8);
+    const double tall = chained(nst, R, high), halved = chained((rows + 511) / 512, 16, low);
+    if(apart <= std::min(tall, halved)) return 0;
+    return tall <= halved ? kRowLong | kRowChain : kRowLong | kRowChain | kRowR16;
 }
 
 static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode, int32_t *d_out, Tiles tiles,
@@ -1831,27 +1835,35 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
         chain_off.assign(K + 1, 0);
         const uint64_t resident = 2 * (uint64_t) ctx->num_sms;
         if(tiles.R == 32 && tiles.W == 8 && !ctx->nw_variant && !ctx->tile_r && long_ok(tbl, gap)) {
-            // A task's time in instructions of one warp: steps times (rows per lane + 28).
+            // A task's time in instructions of one warp: steps times (rows per lane + kStepCost).
             auto task_cost = [&](uint32_t k) {
                 const uint64_t R = strip_rows<32>((int) rows_at(k), 0), nst = (rows_at(k) + 32 * R - 1) / (32 * R);
-                return nst * (cols_at(k) + 31) * (R + 28);
+                return nst * (cols_at(k) + 31) * (R + kStepCost);
             };
             uint64_t total = 0;
             for(uint32_t k = k_lo; k < k_hi; ++k) total += groups_k[k] * task_cost(k);
             uint32_t kc = k_lo;
-            uint64_t groups = 0, strips = 0, low = 0;
+            double high = 0, low = 0;
             for(; kc < k_hi; ++kc) {
                 const uint64_t rows = rows_at(kc), words = groups_k[kc] * 8 * chain_words_of((uint32_t) eff_at(2 * kc + 1));
                 if(rows <= 32 * 32 || !row_narrow[kc] || (kc == k_lo ? 1 : 2) * resident * task_cost(kc) < total) break;
                 if(chain_words + words > (kChainBytes >> 2)) break;
                 chain_off[kc] = chain_words;
                 chain_words += words;
-                groups += groups_k[kc];
-                strips += groups_k[kc] * ((rows + 1023) / 1024);
-                low += groups_k[kc] * ((rows + 511) / 512);
+                const double steps = (double) (groups_k[kc] * (cols_at(kc) + 31));
+                const uint64_t R = strip_rows<32>((int) rows, 0);
+                high += steps * (double) ((rows + 1023) / 1024 * (R + kStepCost + kMovingCost));
+                low += steps * (double) ((rows + 511) / 512 * (16 + kStepCost + kMovingCost));
             }
-            const uint8_t form = kc == k_lo ? 0 : chain_form(rows_at(k_lo), cols_at(k_lo), row_narrow[k_lo] & kRowLong, groups,
-                                                             strips, low, resident);
+            uint8_t form = 0;
+            if(kc > k_lo) {
+                const double steps = (double) (cols_at(k_lo) + 31);
+                const uint64_t R = strip_rows<32>((int) rows_at(k_lo), 0);
+                form = chain_form(rows_at(k_lo), cols_at(k_lo), row_narrow[k_lo] & kRowLong,
+                                  (double) total / (double) task_cost(k_lo),
+                                  high / (steps * (double) (R + kStepCost + kMovingCost)),
+                                  low / (steps * (double) (16 + kStepCost + kMovingCost)), (double) resident);
+            }
             if(!(form & kRowChain)) {
                 kc = k_lo;
                 chain_words = 0;

@@ -1795,20 +1795,37 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
             groups_k[k] = (uint64_t) (ncol + tiles.W - 1) / tiles.W;
             if(nar && k >= k_lo && k < k_hi) pl->narrow_tasks += (uint32_t) groups_k[k];
         }
+        const uint64_t resident = 2 * (uint64_t) ctx->num_sms;
+        // A task's time in instructions of one warp: steps times (rows per lane + kStepCost).
+        auto task_cost = [&](uint32_t k) {
+            const uint64_t R = strip_rows<32>((int) rows_at(k), 0), nst = (rows_at(k) + 32 * R - 1) / (32 * R);
+            return nst * (cols_at(k) + 31) * (R + kStepCost);
+        };
         // Short rows pairs stacked in one warp (stack_task), four by four up to
         // 256 rows and two by two up to 512: all on 16-bit lanes with the state
         // bound holding for 512 rows, the first's longer sequence within the
         // lanes, the last with two sequences and columns, and all in this
-        // part. The others' tasks are the first's. Stacking leaves fewer tasks,
-        // so it is used where at least two per resident CTA are left (120
-        // proteins of 80 to 600 residues: 172 us stacked two by two, 143 us not;
-        // 257 of 150 to 400: 274 us stacked, 350 us not).
+        // part. The others' tasks are the first's. Stacking leaves fewer and
+        // longer tasks, so it is used where at least two per resident CTA are
+        // left (257 proteins of 150 to 400 residues: 274 us stacked two by two,
+        // 350 us not), and two by two also where the tasks are more than the
+        // resident CTAs, none stands out and all can be stacked, since then a
+        // second round of them costs more: stacked against not, 100 proteins of 20 residues 45 and 50
+        // us, of 100 to 150 56 and 67, of 300 to 400 122 and 136, 170 of 200 to
+        // 256 122 and 157. 120 of 80 to 600, whose mean task is 0.63 of the
+        // longest: 153 and 141; 100 of 480 to 600: 261 and 206; 64 of 100 to 150,
+        // one round: 56 and 55.
         if(tiles.R == 32 && narrow_ok(512, 512, tbl, gap)) {
-            uint64_t groups_all = 0;
-            for(uint32_t k = k_lo; k < k_hi; ++k) groups_all += groups_k[k];
-            const uint64_t fill = 4 * (uint64_t) ctx->num_sms;   // twice the resident CTAs
+            uint64_t groups_all = 0, total = 0, longest = 0;
+            for(uint32_t k = k_lo; k < k_hi; ++k) {
+                groups_all += groups_k[k];
+                total += groups_k[k] * task_cost(k);
+                longest = std::max(longest, task_cost(k));
+            }
+            const uint64_t fill = 2 * resident;
+            const bool even = groups_all > resident && 10 * total >= 7 * longest * groups_all && rows_at(k_lo) <= 16 * 32;
             auto stack = [&](uint32_t pairs, uint32_t rows, uint8_t flag) {
-                if(groups_all < pairs * fill) return;
+                if(groups_all < pairs * fill && !(pairs == 2 && even)) return;
                 for(uint32_t k = k_lo; k + pairs <= k_hi;) {
                     bool ok = 2 * ((uint64_t) k + pairs) <= nrows;
                     for(uint32_t p = 0; p < pairs; ++p)
@@ -1833,13 +1850,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
         // below it, the order of the tasks balances them, and chaining would
         // cost 1,200 uneven sequences 0.3%.)
         chain_off.assign(K + 1, 0);
-        const uint64_t resident = 2 * (uint64_t) ctx->num_sms;
         if(tiles.R == 32 && tiles.W == 8 && !ctx->nw_variant && !ctx->tile_r && long_ok(tbl, gap)) {
-            // A task's time in instructions of one warp: steps times (rows per lane + kStepCost).
-            auto task_cost = [&](uint32_t k) {
-                const uint64_t R = strip_rows<32>((int) rows_at(k), 0), nst = (rows_at(k) + 32 * R - 1) / (32 * R);
-                return nst * (cols_at(k) + 31) * (R + kStepCost);
-            };
             uint64_t total = 0;
             for(uint32_t k = k_lo; k < k_hi; ++k) total += groups_k[k] * task_cost(k);
             uint32_t kc = k_lo;

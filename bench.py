@@ -287,13 +287,14 @@ def packed_row_fraction(wl, rmax: int = 32) -> float:
     return packed / total if total else 0.0
 
 
-def nw_ceilings(wl, workload: str, nsm: int, sm_mhz: float, lds: float) -> tuple:
+def nw_ceilings(wl, workload: str, nsm: int, sm_mhz: float, lds: float, planes: bool) -> tuple:
     """Ceilings (GCUPS) of the batched kernel on a workload from rates measured
     per SM clock: shared-memory profile reads at 2 - f bytes per cell (f: the
     packed-row share of the cells, from the kernel's plan), the ALU pipe at
     (1 + f) / 2 lane-ops per cell (64 lanes/clk/SM), and issue at the
     lane-instructions per cell that ncu counted for this kernel on this
-    workload (profiles/nw_traffic.json), when there is a count. Returns the
+    workload (profiles/nw_traffic.json), when there is a count; or, where the
+    measured call ran on bit planes (`planes`), of that kernel. Returns the
     ceilings, the binding one, f, the counted instructions per cell and the
     DRAM traffic of one launch."""
     traffic = inst = None
@@ -306,7 +307,7 @@ def nw_ceilings(wl, workload: str, nsm: int, sm_mhz: float, lds: float) -> tuple
         except Exception:
             traffic = inst = None
     f = packed_row_fraction(wl)
-    if wl.table == "default":
+    if planes:
         # Bit planes (nw_bits.cu): eight three-input logic operations on the ALU
         # pipe and one shared-memory word per 32 cells.
         c = {"alu": nsm * (64.0 * 32 / 8) * sm_mhz * 1e6 / 1e9, "smem": nsm * (lds / 4.0 * 32) * sm_mhz * 1e6 / 1e9}
@@ -386,12 +387,13 @@ def side_workload(lib, ctx, stream, name: str, steps: int, plain_steps: int, sm_
     sc = Scorer(lib, ctx, stream, wl, device)
     ms, kms, st = sc.timed(_lib.MSA_NW_PERSISTENT, steps, 3)
     a = sc.out.clone()
+    planes = lib.msa_nw_last_plane_tasks(ctx.handle) > 0
     pms, pkms, _ = sc.timed(_lib.MSA_NW_PLAIN, plain_steps, 1)
     agree = bool(torch.equal(a, sc.out))
     sc.release()
     cells = wl.cells()
     nsm = torch.cuda.get_device_properties(device).multi_processor_count
-    c, bound, f, inst, traffic = nw_ceilings(wl, name, nsm, sm_mhz, lds)
+    c, bound, f, inst, traffic = nw_ceilings(wl, name, nsm, sm_mhz, lds, planes)
     kg = cells / (kms / 1e3) / 1e9
     return {"config": workload_config(name, wl), "value": cells / (ms / 1e3) / 1e9, "unit": "GCUPS",
             "ms_per_step": ms, "steps": steps, "kernel_gcups": kg,
@@ -747,6 +749,7 @@ def shard_bench(args):
     launches0 = ctx.launches
     step_ms = timed_steps(step, args.steps, args.warmup, timer, barrier, maxr)
     launches = (ctx.launches - launches0) // max(args.steps + args.warmup, 1)
+    planes = lib.msa_nw_last_plane_tasks(ctx.handle) > 0
     clocks = sampler.stop()
 
     # Whole matrix on rank 0: checked against the one-device result.
@@ -792,7 +795,7 @@ def shard_bench(args):
         nsm = torch.cuda.get_device_properties(local).multi_processor_count
         sm_mhz = clocks.get("sm_mhz") or 1965.0
         lds = probe_rate(ctx, 15)
-        c, bound, f, inst, traffic = nw_ceilings(wl, args.workload, nsm, sm_mhz, lds)
+        c, bound, f, inst, traffic = nw_ceilings(wl, args.workload, nsm, sm_mhz, lds, planes)
         per_gpu = cfg["cells"] / (step_ms / 1e3) / 1e9 / world
         roof = {"bound": bound, "achieved": per_gpu, "peak": c[bound], "unit": "GCUPS", "frac": per_gpu / c[bound],
                 "traffic": traffic, "ceilings_gcups": c, "packed_row_fraction": f,
@@ -912,6 +915,7 @@ def main():
     sampler = ClockSampler(local)
     sampler.start()
     ms, kms, launches, st = timed(_lib.MSA_NW_PERSISTENT, args.steps, args.warmup)
+    planes = lib.msa_nw_last_plane_tasks(ctx.handle) > 0
     clocks = sampler.stop()
     plain_ms, plain_kms, _, _ = timed(_lib.MSA_NW_PLAIN, args.plain_steps, 1)
 
@@ -972,7 +976,7 @@ def main():
         # lowest one is the roofline.
         lds = probe_rate(ctx, 15)
         cell_ops = probe_rate(ctx, 14)
-        ceilings, bound, f_packed, inst_per_cell, traffic = nw_ceilings(wl, args.workload, nsm, sm_mhz, lds)
+        ceilings, bound, f_packed, inst_per_cell, traffic = nw_ceilings(wl, args.workload, nsm, sm_mhz, lds, planes)
         cell_peak = nsm * (2.0 * cell_ops) * sm_mhz * 1e6 / 1e9
         roof = ceilings[bound]
         # The four-op int32 issue figure (two max operations per cell on the ALU
@@ -1003,7 +1007,7 @@ def main():
                                             "cell_ops_16x2_probe": cell_peak, "int32_issue_4ops_per_cell": peak},
                          "measured_per_sm_clk": {"lds_bytes": lds, "cell_16x2_lane_ops": cell_ops},
                          "peak_basis": (f"{nsm} SM x 64 ALU lanes/clk x 32 cells / 8 logic operations"
-                                        if wl.table == "default" else
+                                        if planes else
                                         f"min of {nsm} SM x {lds:.1f} shared-memory bytes/clk (measured, "
                                         f"ld.shared.v4) / (2 - {f_packed:.3f}) bytes of profile per cell, "
                                         f"{nsm} SM x 64 ALU lanes/clk / ((1 + {f_packed:.3f}) / 2) lane-ops per cell"

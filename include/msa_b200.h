@@ -227,10 +227,14 @@ typedef struct msa_nw_stats {
     uint64_t pairs;
     uint32_t launches;      /* kernel launches issued by the call */
     uint32_t narrow_tasks;  /* tasks whose values fit 16-bit lanes as they are (longer ones run
-                               on 16-bit lanes relative to a moving base, or on 32-bit lanes) */
+                               on 16-bit lanes relative to a moving base, or on 32-bit lanes),
+                               and the tasks on bit planes (msa_nw_last_plane_tasks) */
     uint32_t graph;         /* 1 if the call replayed a captured CUDA graph */
 } msa_nw_stats;
 int msa_nw_last_stats(const msa_ctx *ctx, msa_nw_stats *out);
+/* Tasks of that call that ran on bit planes (tables of one match and one mismatch
+ * score, see nw_bits.cu); 0: none of it did. */
+uint32_t msa_nw_last_plane_tasks(const msa_ctx *ctx);
 
 /*
  * All-pairs NW that allocates nothing (no counterpart in the reference, which

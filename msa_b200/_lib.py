@@ -142,6 +142,7 @@ _PROTOS = [
                               ctypes.POINTER(MsaOtu)]),
     ("msa_nj_order", ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_uint32, ctypes.c_int,
                                     ctypes.POINTER(MsaOtu)]),
+    ("msa_nw_last_plane_tasks", ctypes.c_uint32, [ctypes.c_void_p]),
     ("msa_release_idle", ctypes.c_int, [ctypes.c_void_p]),
     ("msa_nw_set_wait", ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint32]),
     ("msa_nj_last_stats", ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(MsaNjStats)]),

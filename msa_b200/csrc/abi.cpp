@@ -526,6 +526,8 @@ int msa_nw_last_stats(const msa_ctx *ctx, msa_nw_stats *out)
     return MSA_OK;
 }
 
+uint32_t msa_nw_last_plane_tasks(const msa_ctx *ctx) { return ctx ? ctx->last_plane_tasks : 0; }
+
 int msa_nj_set_clusters(msa_ctx *ctx, int clusters, uint32_t helper_min_count, uint32_t wait_limit_us,
                         int stall_publication)
 {

@@ -149,6 +149,7 @@ struct msa_ctx {
     int nj_clusters = 0;
     uint32_t nj_helper_c = 0, nj_wait_us = 0;
     int nj_stall = 0;
+    uint32_t last_plane_tasks = 0;   // of the last call (msa_nw_last_plane_tasks)
     uint32_t nw_wait_us = 0;   // msa_nw_set_wait: limit of the waits between strips (0 = default)
 };
 

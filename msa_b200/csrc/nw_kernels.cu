@@ -2113,6 +2113,7 @@ int nw_run(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode, int32_t *d
     const uint32_t n = st->n;
     msa_nw_stats stats{};
     stats.pairs = (uint64_t) n * (n > 0 ? n - 1 : 0) / 2;
+    ctx->last_plane_tasks = 0;
     if(n < 2) { ctx->last = stats; return MSA_OK; }
 
     const uint32_t nclean = (uint32_t) st->clean_sorted.size();
@@ -2194,6 +2195,7 @@ int nw_run(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode, int32_t *d
     stats.cells = pl->cells;
     stats.launches = pl->launches;
     stats.narrow_tasks = pl->narrow_tasks;
+    ctx->last_plane_tasks = pl->bits.ntasks;
     stats.graph = use_graph ? 1 : 0;
     ctx->last = stats;
     return MSA_OK;

@@ -1545,6 +1545,7 @@ struct NwPlan {
     int variant = 0;            // msa_nw_set_variant flags the plan was built with
     uint32_t chunk = 0;         // and its groups-per-task override
     uint32_t wait_us = 0;       // and its waits (msa_nw_set_wait)
+    bool fixed_tiles = false;   // and whether it says the tiles (msa_nw_set_tiles)
     size_t clear_bytes = 64;    // of the work counter and what follows it
     bool chained = false;
     bool profiles = true;       // whether any kernel of the plan reads score profiles
@@ -1701,6 +1702,7 @@ static int build_plan(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode,
     pl->variant = ctx->nw_variant;
     pl->chunk = ctx->nw_chunk;
     pl->wait_us = ctx->nw_wait_us;
+    pl->fixed_tiles = ctx->tile_r != 0;
 
     const uint32_t nclean = (uint32_t) st->clean_sorted.size();
     const uint64_t nclean_pairs = (uint64_t) nclean * (nclean > 0 ? nclean - 1 : 0) / 2;
@@ -2128,7 +2130,8 @@ int nw_run(msa_ctx *ctx, SeqStore *st, const ExtTable &tbl, int mode, int32_t *d
         NwPlan *c = plans[i];
         if(c->store_serial == st->serial && c->mode == mode && c->d_out == d_out && c->tiles.R == tiles.R &&
            c->tiles.W == tiles.W && c->part == part && c->nparts == nparts && same_table(c->tbl, tbl) &&
-           c->variant == ctx->nw_variant && c->chunk == ctx->nw_chunk && c->wait_us == ctx->nw_wait_us) {
+           c->variant == ctx->nw_variant && c->chunk == ctx->nw_chunk && c->wait_us == ctx->nw_wait_us &&
+           c->fixed_tiles == (ctx->tile_r != 0)) {
             pl = c;
             plans.erase(plans.begin() + i);
             plans.push_back(pl);

@@ -293,11 +293,13 @@ __global__ void __launch_bounds__(128) nw_match_kernel(BitParams p)
 constexpr int kRingWords = kRingRows * 112;
 constexpr size_t kRingBytes = kBitWarps * kRingWords * sizeof(uint32_t);
 
-// Four warps per CTA, four CTAs per SM. With three, and registers to spare, 1,200
-// uneven sequences took 76.5 ms instead of 71.8. A step of R rows is one pass of the
-// loop where R is above 16: two steps to a pass save an addition per row, but
-// the warps' places in the code then outgrow the instruction caches (78.1 ms; four
-// steps 98.6). Every warp takes its own tasks, longest rows first.
+// Four warps per CTA, four CTAs per SM. 1,200 uneven sequences, before the split of a
+// job counted a warp's pace beside three others (65 ms since): with three CTAs, and
+// registers to spare, 76.5 ms instead of 71.8. A step of R rows is one pass of the loop
+// where R is above 16: two steps to a pass save an addition per row, but the warps'
+// places in the code then outgrow the instruction caches (78.1 ms; four steps 98.6).
+// Every warp takes its own tasks, longest rows first. ptxas spills 4 to 52 bytes in the
+// tasks of 22 rows and more.
 __global__ void __launch_bounds__(kBitWarps * 32, 4) nw_bits_kernel(BitParams p)
 {
     extern __shared__ __align__(16) uint32_t rings[];
@@ -313,8 +315,8 @@ __global__ void __launch_bounds__(kBitWarps * 32, 4) nw_bits_kernel(BitParams p)
         }
         return p.sets[lo];
     };
-    // Chained tasks: strip s on warp s mod kBitWarps (1,200 uneven sequences: 117
-    // ms with every task on one warp, 98.6 chained).
+    // Chained tasks: strip s on warp s mod kBitWarps (1,200 uneven sequences, with four
+    // steps to a pass: 117 ms with every task on one warp, 98.6 chained).
     while(p.nchain) {
         __syncthreads();
         if(threadIdx.x == 0) task = atomicAdd(p.counter, 1ull);

@@ -264,7 +264,7 @@ int build_store(msa_ctx *ctx, const uint8_t *units, const uint64_t *offs, const 
         st->prof_lp.resize(n);
         uint64_t poff = 0;
         for(uint32_t i = 0; i < n; ++i) {
-            st->prof_lp[i] = (uint32_t) round_up(std::max<uint32_t>(st->eff[i], 1), kProfPad);
+            st->prof_lp[i] = (uint32_t) prof_pitch(st->eff[i]);
             st->prof_off[i] = poff;
             poff += (uint64_t) kAlpha * st->prof_lp[i];
         }

@@ -19,12 +19,17 @@ namespace msa {
 
 // Profile rows: encoder units 0..25 (24 = END never scored, 25 = GAP).
 constexpr int kAlpha = 26;
-// Profile rows are padded to a multiple of the tallest strip (32 lanes x 32 rows).
+// Profile rows are padded to a multiple of the tallest strip (32 lanes x 32 rows; prof_pitch).
 constexpr int kProfPad = 1024;
 // Every sequence's units are padded with END so 16-byte loads past the end stay in bounds.
 constexpr int kUnitPad = 64;
 
 inline uint64_t round_up(uint64_t x, uint64_t m) { return (x + m - 1) / m * m; }
+
+// Rows of the score profile of a sequence of `eff` units: those of the strips of a
+// rows pair in which it is the first. Where the reference's orientation decides, the
+// second has as many 3-unit blocks and may be up to two rows longer.
+inline uint64_t prof_pitch(uint64_t eff) { return round_up((eff ? eff : 1) + 2, kProfPad); }
 
 // Built-in tables in storage order (tables.inc).
 struct BuiltinTable {
@@ -71,7 +76,7 @@ struct SeqStore {
     // Clean sequences, longest first (order_clean).
     std::vector<uint32_t> clean_sorted;
     uint32_t *d_clean_sorted = nullptr;
-    // Profile geometry per sequence (original index): Lp = round_up(max(eff,1), kProfPad).
+    // Profile geometry per sequence (original index): Lp = prof_pitch(eff).
     std::vector<uint64_t> prof_off;
     std::vector<uint32_t> prof_lp;
     uint64_t prof_bytes = 0;

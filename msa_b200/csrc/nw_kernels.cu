@@ -451,16 +451,14 @@ __device__ __forceinline__ uint32_t prmt0(uint32_t w)
 
 // Stages strip rows [i0, i0 + 32R) of the profile in shared memory (Layout).
 // Narrow: word = (s(X1_i, b) + 2g, s(X2_i, b) + 2g) as 16x2 (see Narrow), or
-// bytes (s1_i, s1_i+1, s2_i, s2_i+1) + 2g in the packed planes; rows past a
-// sequence's profile (lp1, lp2) score 0: either may be the longer one where the
-// reference's orientation decides (1,024 and 1,026 rows are one length in blocks of
-// three, and one of them has a strip more). Wide: word = s(X1_i, b) as int32.
+// bytes (s1_i, s1_i+1, s2_i, s2_i+1) + 2g in the packed planes; rows of X2 past
+// its profile (lp2) score 0, X1's reaches as far as the strips (prof_pitch). Wide: word = s(X1_i, b) as int32.
 // The profile is read in 16-byte chunks (16 rows of one code), each thread
 // issuing the loads of up to kStageBatch chunks before it converts and stores
 // any, so one staging costs about one L2 round trip instead of one per chunk.
 // Profile rows are 16-byte aligned: the per-sequence pitch is a multiple of
-// 1024 and i0 a multiple of 64; lp1 and lp2 are multiples of 1024, so a chunk lies
-// wholly inside or wholly past a profile. Stacked rows pairs have at most 512 rows.
+// 1024 and i0 a multiple of 64; lp2 is a multiple of 1024, so a chunk lies
+// wholly inside or wholly past X2's profile. Stacked rows pairs have at most 512 rows.
 constexpr int kStageBatch = 4;
 
 // A rows pair's score profiles as staging reads them.
@@ -493,8 +491,7 @@ __device__ __forceinline__ void stage_words(uint32_t *sprof, const int8_t *__res
                 if(c < TOTAL) {
                     const int b = c / CH, m = c - b * CH;
                     if constexpr(kPairs == 1) {
-                        if((uint32_t) (i0 + 16 * m) < lp1)
-                            va[u] = __ldg(reinterpret_cast<const uint4 *>(g1 + (size_t) b * lp1 + i0) + m);
+                        va[u] = __ldg(reinterpret_cast<const uint4 *>(g1 + (size_t) b * lp1 + i0) + m);
                         if((uint32_t) (i0 + 16 * m) < lp2)
                             vb[u] = __ldg(reinterpret_cast<const uint4 *>(g2 + (size_t) b * lp2 + i0) + m);
                     } else {

@@ -291,7 +291,7 @@ uint64_t estimate_bytes(const Job *j)
     uint64_t units = 0, prof = 0;
     for(uint32_t i = 0; i < j->n; ++i) {
         units += round_up(j->lens[i] + 2 + kUnitPad, 16);
-        prof += (uint64_t) kAlpha * round_up(std::max<uint64_t>(j->lens[i], 1), kProfPad);
+        prof += (uint64_t) kAlpha * prof_pitch(j->lens[i]);
     }
     return units + prof + (uint64_t) j->n * (j->n > 0 ? j->n - 1 : 0) * 2 + (uint64_t) j->n * 40 + 4096;
 }
